@@ -1,0 +1,362 @@
+// unet_conv.cuh -- the 3 x 3 x 3 convolutions of the initial-guess network as
+// implicit GEMMs on the sm_100a tensor cores (tcgen05): forward, and the data
+// gradient.  No column matrix: a block brings the voxels of its tile with a
+// one-voxel halo into shared memory once, and every tap's operand is the same
+// memory read from a shifted start address.
+//
+// Activations are stored in planes of 8 channels, [C/8][Vp][8] BF16 (16 bytes
+// per voxel and plane, x fastest).  A tile is 8 x 16 voxels of BZ z-planes; one
+// 4-D TMA box (10 x 8 channels, 18, BZ + 2, C/8) lands as [C/8][z][y][x][8], zero
+// outside the volume.  In it 8 voxels of a row are 128 contiguous bytes -- an
+// unswizzled K-major core matrix (8 rows x 16 bytes) -- rows lie 160 bytes apart
+// (the stride between the 16 core matrices of the 128-row operand) and the
+// planes of 8 channels a fixed stride apart (the two core matrices of K = 16),
+// so the operand of tap (dx, dy, dz) starts 16 dx + 160 dy + 2880 dz bytes on.
+//
+// What bounds them: each K = 16 step reads 4 KB of operand A from shared memory
+// (32 cycles at 128 B per cycle) for 128 x 16 to 128 x 128 outputs, and the tile
+// comes in once instead of 27 times.  The column matrix of the same layers cost
+// 27 x the activations in and out of memory; see conv_fwd for the figures.
+//
+// Every wait is bounded: one that gives up sets the error flag, the later ones
+// are skipped, and the kernel still frees its tensor memory before it returns.
+#pragma once
+#include "unet_gemm.cuh"
+
+namespace aphid {
+namespace unet {
+
+constexpr int kTX = 8, kTY = 16, kRowB = (kTX + 2) * 16, kPlaneB = (kTY + 2) * kRowB;  // tile, bytes of a staged row, plane
+constexpr int kConvThreads = 192;  // warps 0-3: epilogue, 4: producer, 5: MMA issuer
+constexpr int kMaxStages = 4;
+
+struct ConvArgs {
+  int X, Y, Z;         // volume
+  long long Vp;        // voxels per plane of 8 channels
+  int ch;              // 8-channel planes of the input
+  int bz;              // z-planes per tile
+  int tx, ty;          // tiles along x, y
+  int chunks;          // K chunks (8 channels of one tap) in the weight stream, even
+  int per_stage;       // chunks per weight stage, even (forward); taps per stage (data gradient)
+  int stages;          // weight stages
+  unsigned chunk_b;    // bytes of a weight chunk: outputs x 16 (forward); of a tap (data gradient)
+};
+
+// shared-memory descriptor of an unswizzled K-major operand: lbo between the
+// two core matrices of K = 16, sbo between 8-row core matrices (bytes)
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46);
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void g_mbar_init_n(uint32_t bar, uint32_t n) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(n) : "memory");
+}
+__device__ __forceinline__ void g_mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+// 1-D bulk copy into this block's shared memory (16-byte multiples)
+__device__ __forceinline__ void g_bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void g_tma_load4(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int c, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];\n" ::"r"(dst),
+      "l"((unsigned long long)map), "r"(x), "r"(y), "r"(z), "r"(c), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t a, float *x) {
+  uint32_t v[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(a));
+#pragma unroll
+  for (int q = 0; q < 8; q++) x[q] = __uint_as_float(v[q]);
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+
+// shared memory: the input tile, the weight stages, the barriers
+// (with one plane of 8 channels the last K = 16 step has no second tap: its
+// operand is a plane of zeros behind the tile, not a neighbour's value times a
+// zero weight, which an infinity would turn into NaN)
+__host__ __device__ constexpr size_t conv_tile_bytes(int ch, int bz) {
+  return ((size_t)(ch * (bz + 2) + (ch & 1)) * kPlaneB + 127) / 128 * 128;
+}
+inline size_t conv_shm(const ConvArgs &a) {
+  return 128 + conv_tile_bytes(a.ch, a.bz) + (size_t)a.stages * (a.per_stage * a.chunk_b) + 256;
+}
+
+struct ConvShm {
+  unsigned char *tile, *w;
+  uint64_t *full, *empty, *tile_in, *tfull, *tempty;  // [kMaxStages] x 2, 1, 2, 2
+  uint32_t *tslot;
+};
+// carve the dynamic shared memory, allocate `cols` of tensor memory, arm the barriers
+__device__ __forceinline__ ConvShm conv_init(unsigned char *raw, const ConvArgs &a, uint32_t cols, uint32_t &tmem) {
+  ConvShm s;
+  s.tile = raw + ((128u - (gsm(raw) & 127u)) & 127u);
+  s.w = s.tile + conv_tile_bytes(a.ch, a.bz);
+  s.full = reinterpret_cast<uint64_t *>(s.w + (size_t)a.stages * (a.per_stage * a.chunk_b));
+  s.empty = s.full + kMaxStages;
+  s.tile_in = s.empty + kMaxStages;
+  s.tfull = s.tile_in + 1;
+  s.tempty = s.tfull + 2;
+  s.tslot = reinterpret_cast<uint32_t *>(s.tempty + 2);
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(gsm(s.tslot)), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (threadIdx.x == 32) {
+    for (int q = 0; q < kMaxStages; q++) {
+      g_mbar_init(gsm(&s.full[q]));
+      g_mbar_init(gsm(&s.empty[q]));
+    }
+    g_mbar_init(gsm(s.tile_in));
+    for (int q = 0; q < 2; q++) {
+      g_mbar_init(gsm(&s.tfull[q]));
+      g_mbar_init_n(gsm(&s.tempty[q]), 4);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  }
+  if (a.ch & 1) {
+    uint4 *z = reinterpret_cast<uint4 *>(s.tile + (size_t)a.ch * (a.bz + 2) * kPlaneB);
+    for (int q = threadIdx.x; q < kPlaneB / 16; q += kConvThreads) z[q] = make_uint4(0, 0, 0, 0);
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  tmem = *s.tslot;
+  return s;
+}
+__device__ __forceinline__ void conv_exit(uint32_t tmem, uint32_t cols) {
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(cols) : "memory");
+}
+__host__ __device__ constexpr uint32_t tmem_cols(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512; }
+
+// Forward: out = act(conv(in) + bias), BN output channels, BZ z-planes per
+// block.  Weights: the stream [K chunk][BN][8] (K = tap x channels, in that
+// order), read once per block through a ring.  The products are added in the
+// order of K, 16 at a time.  RELU: BF16 planes of 8 channels; else FP32 rows
+// [Vp][BN] (the head).
+template <int BN, int BZ, bool RELU>
+__global__ void __launch_bounds__(kConvThreads) k_conv_fwd(const __grid_constant__ CUtensorMap map, const ConvArgs a,
+                                                           const __nv_bfloat16 *__restrict__ wgt,
+                                                           const float *__restrict__ bias, void *__restrict__ out, int *err) {
+  extern __shared__ unsigned char cs_raw[];
+  constexpr uint32_t kCols = tmem_cols(BN * BZ);
+  uint32_t tmem;
+  const ConvShm s = conv_init(cs_raw, a, kCols, tmem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int b = blockIdx.x;
+  const int x0 = b % a.tx * kTX;
+  b /= a.tx;
+  const int y0 = b % a.ty * kTY, z0 = b / a.ty * BZ;
+  const int nst = (a.chunks + a.per_stage - 1) / a.per_stage;
+  const uint32_t stage_b = a.per_stage * a.chunk_b, plane_b = (BZ + 2) * kPlaneB;
+  bool ok = true;
+  if (warp == 4 && lane == 0) {
+    g_mbar_expect(gsm(s.tile_in), (uint32_t)a.ch * plane_b);
+    g_tma_load4(gsm(s.tile), &map, (x0 - 1) * 8, y0 - 1, z0 - 1, 0, gsm(s.tile_in));
+    for (int q = 0; q < nst; q++) {
+      const int st = q % a.stages;
+      if (q >= a.stages && ok) ok = g_mbar_wait(gsm(&s.empty[st]), (uint32_t)((q / a.stages - 1) & 1));
+      const uint32_t bytes = min(a.per_stage, a.chunks - q * a.per_stage) * a.chunk_b;
+      g_mbar_expect(gsm(&s.full[st]), bytes);
+      g_bulk_load(gsm(s.w) + st * stage_b, wgt + (size_t)q * stage_b / 2, bytes, gsm(&s.full[st]));
+    }
+  } else if (warp == 5 && lane == 0) {
+    constexpr uint32_t idesc = idesc_bf16(kBM, BN);
+    ok = g_mbar_wait(gsm(s.tile_in), 0u);
+    const uint32_t tile = gsm(s.tile);
+    auto tap_at = [](int t) { return (uint32_t)(t % 3 * 16 + t / 3 % 3 * kRowB + t / 9 * kPlaneB); };
+    for (int q = 0; q < nst; q++) {
+      const int st = q % a.stages;
+      if (ok) ok = g_mbar_wait(gsm(&s.full[st]), (uint32_t)((q / a.stages) & 1));
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const int k1 = min(a.chunks, (q + 1) * a.per_stage);
+      for (int k = q * a.per_stage; k < k1; k += 2) {
+        const int t = k / a.ch, c = k - t * a.ch;
+        // K = 16: two planes of one tap, or (one plane) two taps, the last with zeros
+        const uint32_t at = tap_at(t);
+        const uint64_t db = smem_desc(gsm(s.w) + st * stage_b + (k - q * a.per_stage) * a.chunk_b, a.chunk_b, 128);
+        const uint32_t a0 = tile + c * plane_b + at;
+#pragma unroll
+        for (int p = 0; p < BZ; p++) {
+          const uint32_t lbo = a.ch > 1 ? plane_b : t < 26 ? tap_at(t + 1) - at : plane_b - at - p * kPlaneB;
+          mma_f16(tmem + p * BN, smem_desc(a0 + p * kPlaneB, lbo, kRowB), db, idesc, k > 0);
+        }
+      }
+      mma_commit(gsm(&s.empty[st]));
+    }
+    mma_commit(gsm(s.tfull));
+  }
+  __syncwarp();
+  if (warp < 4) {
+    ok = g_mbar_wait(gsm(s.tfull), 0u) && ok;
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    // lane = row of the tile: x fastest
+    const int x = x0 + (lane & 7), y = y0 + warp * 4 + (lane >> 3);
+    const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+    for (int p = 0; p < BZ; p++) {
+      const int z = z0 + p;
+      const long long v = x + (long long)a.X * (y + (long long)a.Y * z);
+      const bool in = x < a.X && y < a.Y && z < a.Z;
+#pragma unroll
+      for (int c0 = 0; c0 < BN; c0 += 16) {
+        float f[16];
+        __syncwarp();
+        tmem_ld8(acc + p * BN + c0, f);
+        tmem_ld8(acc + p * BN + c0 + 8, f + 8);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 16; q++) f[q] += __ldg(bias + c0 + q);
+        if (in && RELU) {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            uint32_t u[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+              u[q] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(fmaxf(f[8 * h + 2 * q], 0.f))) |
+                     ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(fmaxf(f[8 * h + 2 * q + 1], 0.f))) << 16);
+            reinterpret_cast<uint4 *>(out)[(c0 / 8 + h) * a.Vp + v] = make_uint4(u[0], u[1], u[2], u[3]);
+          }
+        } else if (in) {
+          float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + v * BN + c0);
+#pragma unroll
+          for (int q = 0; q < 4; q++) o[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+        }
+      }
+    }
+  }
+  if (!ok && err) atomicExch(err, 1);
+  conv_exit(tmem, kCols);
+}
+
+// Data gradient: gin[u][c] += sum over the taps t = 0 .. 26 of
+// sum_co dz[u - d_t][co] W[co][t][c], NC input channels of group blockIdx.y, BZ
+// z-planes per block.  Each tap's products are formed in tensor memory on their
+// own and added in FP32 registers in the order of the taps, as a column matrix
+// and its gather would add them: a sum over the taps inside tensor memory would
+// round differently, and the next layer's BF16 rounding turns that into steps.
+// Two tensor-memory buffers: the tap after the one being added is in flight.
+// Weights: [group][tap][co / 8][NC][8].
+template <int NC, int BZ>
+__global__ void __launch_bounds__(kConvThreads) k_conv_dx(const __grid_constant__ CUtensorMap map, const ConvArgs a,
+                                                          const __nv_bfloat16 *__restrict__ wgt, int C,
+                                                          float *__restrict__ gin, int *err) {
+  extern __shared__ unsigned char cs_raw[];
+  constexpr uint32_t kCols = tmem_cols(2 * NC * BZ);
+  uint32_t tmem;
+  const ConvShm s = conv_init(cs_raw, a, kCols, tmem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int b = blockIdx.x;
+  const int x0 = b % a.tx * kTX;
+  b /= a.tx;
+  const int y0 = b % a.ty * kTY, z0 = b / a.ty * BZ;
+  constexpr int kTaps = 27;
+  const int nst = (kTaps + a.per_stage - 1) / a.per_stage;
+  const uint32_t stage_b = a.per_stage * a.chunk_b, plane_b = (BZ + 2) * kPlaneB;
+  bool ok = true;
+  if (warp == 4 && lane == 0) {
+    const __nv_bfloat16 *w = wgt + (size_t)blockIdx.y * kTaps * a.chunk_b / 2;
+    g_mbar_expect(gsm(s.tile_in), (uint32_t)a.ch * plane_b);
+    g_tma_load4(gsm(s.tile), &map, (x0 - 1) * 8, y0 - 1, z0 - 1, 0, gsm(s.tile_in));
+    for (int q = 0; q < nst; q++) {
+      const int st = q % a.stages;
+      if (q >= a.stages && ok) ok = g_mbar_wait(gsm(&s.empty[st]), (uint32_t)((q / a.stages - 1) & 1));
+      const uint32_t bytes = min(a.per_stage, kTaps - q * a.per_stage) * a.chunk_b;
+      g_mbar_expect(gsm(&s.full[st]), bytes);
+      g_bulk_load(gsm(s.w) + st * stage_b, w + (size_t)q * stage_b / 2, bytes, gsm(&s.full[st]));
+    }
+  } else if (warp == 5 && lane == 0) {
+    constexpr uint32_t idesc = idesc_bf16(kBM, NC);
+    ok = g_mbar_wait(gsm(s.tile_in), 0u);
+    const uint32_t tile = gsm(s.tile);
+    for (int t = 0; t < kTaps; t++) {
+      const int q = t / a.per_stage, st = q % a.stages, buf = t & 1;
+      if (t == q * a.per_stage && ok) ok = g_mbar_wait(gsm(&s.full[st]), (uint32_t)((q / a.stages) & 1));
+      if (t >= 2 && ok) ok = g_mbar_wait(gsm(&s.tempty[buf]), (uint32_t)((t / 2 - 1) & 1));
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      // u - d_t: the staged voxel 1 - d_t on
+      const uint32_t at = (uint32_t)((2 - t % 3) * 16 + (2 - t / 3 % 3) * kRowB + (2 - t / 9) * kPlaneB);
+      const uint32_t w0 = gsm(s.w) + st * stage_b + (t - q * a.per_stage) * a.chunk_b;
+      for (int c = 0; c < a.ch; c += 2) {
+        const uint64_t db = smem_desc(w0 + c * (NC * 16), NC * 16, 128);
+        const uint32_t a0 = tile + c * plane_b + at;
+#pragma unroll
+        for (int p = 0; p < BZ; p++)
+          mma_f16(tmem + (buf * BZ + p) * NC, smem_desc(a0 + p * kPlaneB, plane_b, kRowB), db, idesc, c > 0);
+      }
+      mma_commit(gsm(&s.tfull[buf]));
+      if (t + 1 == kTaps || (t + 1) % a.per_stage == 0) mma_commit(gsm(&s.empty[st]));
+    }
+  }
+  __syncwarp();
+  if (warp < 4) {
+    float sum[BZ * NC];
+#pragma unroll
+    for (int q = 0; q < BZ * NC; q++) sum[q] = 0.f;
+    const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+    for (int t = 0; t < kTaps; t++) {
+      const int buf = t & 1;
+      if (ok) ok = g_mbar_wait(gsm(&s.tfull[buf]), (uint32_t)((t / 2) & 1));
+      __syncwarp();
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+      for (int q = 0; q < BZ * NC; q += 16) {
+        float f[16];
+        tmem_ld8(acc + buf * BZ * NC + q, f);
+        tmem_ld8(acc + buf * BZ * NC + q + 8, f + 8);
+        tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < 16; h++) sum[q + h] += f[h];
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) g_mbar_arrive(gsm(&s.tempty[buf]));
+    }
+    const int x = x0 + (lane & 7), y = y0 + warp * 4 + (lane >> 3);
+#pragma unroll
+    for (int p = 0; p < BZ; p++) {
+      const int z = z0 + p;
+      if (x >= a.X || y >= a.Y || z >= a.Z) continue;
+      const long long v = x + (long long)a.X * (y + (long long)a.Y * z);
+      float4 *g = reinterpret_cast<float4 *>(gin + v * C + (int)blockIdx.y * NC);
+#pragma unroll
+      for (int q = 0; q < NC / 4; q++) {
+        float4 o = g[q];
+        o.x += sum[p * NC + 4 * q];
+        o.y += sum[p * NC + 4 * q + 1];
+        o.z += sum[p * NC + 4 * q + 2];
+        o.w += sum[p * NC + 4 * q + 3];
+        g[q] = o;
+      }
+    }
+  }
+  if (!ok && err) atomicExch(err, 1);
+  conv_exit(tmem, kCols);
+}
+
+}  // namespace unet
+}  // namespace aphid
