@@ -522,64 +522,75 @@ int act_map(CUtensorMap *m, const __nv_bfloat16 *base, int C, const Vol &v, int 
   if (r != CUDA_SUCCESS) return set_err(APHID_UNET_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
   return APHID_UNET_OK;
 }
-// geometry of a convolution over C input channels of v, units of `unit` weight
-// chunks (2 chunks of K = 8 forward, a tap in the data gradient) of chunk_b bytes
-ConvArgs conv_args(const Vol &v, int C, int bz, int chunks, int unit, int chunk_b) {
-  ConvArgs a{};
-  a.X = v.X, a.Y = v.Y, a.Z = v.Z, a.Vp = v.Vp;
-  a.ch = C / 8, a.bz = bz;
-  a.tx = (v.X + kTX - 1) / kTX, a.ty = (v.Y + kTY - 1) / kTY;
-  a.chunks = chunks, a.chunk_b = (unsigned)chunk_b;
-  // weight stages of about 8 KB, four of them (two beside the largest tiles);
-  // streams of up to 16 KB in one piece
-  a.per_stage = chunks * chunk_b <= 16384 ? chunks : std::max(unit, 8192 / chunk_b / unit * unit);
-  a.stages = std::min((chunks + a.per_stage - 1) / a.per_stage, conv_tile_bytes(a.ch, bz) > 120000 ? 2 : kMaxStages);
-  return a;
+template <class Kernel, class... Args>
+int launch_conv(Kernel kernel, const __nv_bfloat16 *in, int C, const Vol &v, int bz, int groups, size_t shm, cudaStream_t st,
+                Args... args) {
+  ConvArgs a{v.X, v.Y, v.Z, v.Vp, (v.X + kTX - 1) / kTX, (v.Y + kTY - 1) / kTY};
+  CUtensorMap m;
+  UR(act_map(&m, in, C, v, bz));
+  UK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+  kernel<<<dim3((unsigned)(a.tx * a.ty * ((v.Z + bz - 1) / bz)), (unsigned)groups), kConvThreads, shm, st>>>(m, a, args...);
+  UK(cudaGetLastError());
+  return APHID_UNET_OK;
 }
-template <int BN, int BZ, bool RELU>
+template <int CH, int BN, int BZ, int PER, int ST, bool RELU = true>
 int conv_fwd_t(aphid_unet *n, const Layer &l, const __nv_bfloat16 *in, void *out, cudaStream_t st) {
-  const Vol &v = n->vol[l.level];
-  const ConvArgs a = conv_args(v, l.cg, BZ, (27 * (l.cg / 8) + 1) / 2 * 2, 2, BN * 16);
-  CUtensorMap m;
-  UR(act_map(&m, in, l.cg, v, BZ));
-  UK(cudaFuncSetAttribute(k_conv_fwd<BN, BZ, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)conv_shm(a)));
-  k_conv_fwd<BN, BZ, RELU><<<(unsigned)(a.tx * a.ty * ((v.Z + BZ - 1) / BZ)), kConvThreads, conv_shm(a), st>>>(
-      m, a, l.Wf, l.b, out, n->err);
-  UK(cudaGetLastError());
-  return APHID_UNET_OK;
+  return launch_conv(k_conv_fwd<CH, BN, BZ, PER, ST, RELU>, in, CH * 8, n->vol[l.level], BZ, 1,
+                     conv_shm(CH, BZ, ST * PER * BN * 16), st, l.Wf, l.b, out, n->err);
 }
-template <int NC, int BZ>
+template <int CH, int NC, int BZ, int PER, int ST>
 int conv_dx_t(aphid_unet *n, const Layer &l, float *gin, cudaStream_t st) {
-  const Vol &v = n->vol[l.level];
-  const ConvArgs a = conv_args(v, l.cn, BZ, 27, 1, l.cn / 8 * NC * 16);
-  CUtensorMap m;
-  UR(act_map(&m, n->dZ, l.cn, v, BZ));
-  UK(cudaFuncSetAttribute(k_conv_dx<NC, BZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)conv_shm(a)));
-  k_conv_dx<NC, BZ><<<dim3((unsigned)(a.tx * a.ty * ((v.Z + BZ - 1) / BZ)), (unsigned)(l.cg / NC)), kConvThreads,
-                      conv_shm(a), st>>>(m, a, l.Wd, l.cg, gin, n->err);
-  UK(cudaGetLastError());
-  return APHID_UNET_OK;
+  return launch_conv(k_conv_dx<CH, NC, BZ, PER, ST>, n->dZ, CH * 8, n->vol[l.level], BZ, l.cg / NC,
+                     conv_shm(CH, BZ, ST * PER * CH * NC * 16), st, l.Wd, l.cg, gin, n->err);
 }
 
-// One convolution of the forward pass.  z-planes per block: as many as keep
-// the tile near 100 KB (two or three blocks per SM overlap one block's copy
-// with the others' products) and the accumulators within 128 columns.
-// A forward pass of the 161 x 161 x 129 volume takes 4.3 ms with these kernels;
-// with a column matrix and a GEMM per layer it took 22.9 ms, 14.9 of them in
-// writing the column matrices.  A training step of 65 x 65 x 49 takes 5.1 ms
-// (10.8 to 14.2 with column matrices in both directions).  The outputs are the
-// same bit for bit: the order of the products and of the taps is the same.
+// One convolution of the forward pass.  The z-planes per block and the weight
+// stages are the fastest of a sweep over both at the levels of a 168 x 168 x 136
+// and a 72 x 72 x 56 volume: deep tiles save halo and weight traffic while two
+// blocks still fit an SM (one block's copies run under the other's products).
+// Per layer of the larger volume, before -> after the issuing warp's loop and
+// these tiles: 48 -> 16 channels 1468 -> 479 us (4 planes; 1 to 8: 479 to 572),
+// 96 -> 32 654 -> 183 (1 to 4: 285 to 183), 192 -> 64 376 -> 115, 16 -> 16
+// 175 -> 130, 128 -> 128 54 -> 20.
+// A forward pass of the 161 x 161 x 129 volume took 22.9 ms with a column
+// matrix and a GEMM per layer, 14.9 of them in writing the column matrices.  The
+// outputs are the same bit for bit: so is the order of the products.
 int conv_fwd(aphid_unet *n, int li, cudaStream_t st) {
   const Layer &l = n->L[li];
   const __nv_bfloat16 *in = n->act[kLayerIO[li][0]];
-  if (kLayerIO[li][1] < 0) return conv_fwd_t<16, 8, false>(n, l, in, n->y, st);
+  if (kLayerIO[li][1] < 0) return conv_fwd_t<2, 16, 4, 54, 1, false>(n, l, in, n->y, st);
   __nv_bfloat16 *out = n->act[kLayerIO[li][1]];
-  switch (l.cn) {
-    case 16: return l.cg <= 16 ? conv_fwd_t<16, 8, true>(n, l, in, out, st) : conv_fwd_t<16, 4, true>(n, l, in, out, st);
-    case 32: return l.cg <= 32 ? conv_fwd_t<32, 4, true>(n, l, in, out, st) : conv_fwd_t<32, 2, true>(n, l, in, out, st);
-    case 64: return l.cg <= 64 ? conv_fwd_t<64, 2, true>(n, l, in, out, st) : conv_fwd_t<64, 1, true>(n, l, in, out, st);
-    default: return conv_fwd_t<128, 1, true>(n, l, in, out, st);
+  switch (l.cg * 1000 + l.cn) {
+    case 8016: return conv_fwd_t<1, 16, 4, 28, 1>(n, l, in, out, st);
+    case 16016: return conv_fwd_t<2, 16, 4, 54, 1>(n, l, in, out, st);
+    case 16032: return conv_fwd_t<2, 32, 2, 18, 2>(n, l, in, out, st);
+    case 32032: return conv_fwd_t<4, 32, 2, 12, 4>(n, l, in, out, st);
+    case 32064: return conv_fwd_t<4, 64, 1, 12, 2>(n, l, in, out, st);
+    case 64064: return conv_fwd_t<8, 64, 1, 8, 4>(n, l, in, out, st);
+    case 64128: return conv_fwd_t<8, 128, 1, 8, 4>(n, l, in, out, st);
+    case 128128: return conv_fwd_t<16, 128, 1, 8, 4>(n, l, in, out, st);
+    case 192064: return conv_fwd_t<24, 64, 1, 8, 2>(n, l, in, out, st);
+    case 96032: return conv_fwd_t<12, 32, 4, 12, 2>(n, l, in, out, st);
+    case 48016: return conv_fwd_t<6, 16, 4, 18, 2>(n, l, in, out, st);
   }
+  return set_err(APHID_UNET_ERR_BADARG, "no convolution kernel for this layer");
+}
+
+// The data gradient of one layer into gin.  Few planes per block here: the
+// epilogue's sums take BZ x NC registers, and three or four blocks per SM hide
+// its reads of tensor memory (a 72 x 72 x 56 volume, 16 -> 16 channels: 25, 31,
+// 37 us at 2, 4, 8 planes; 32 of 96 channels at half of it: 33, 46 at 1, 2).
+int conv_dx(aphid_unet *n, int li, float *gin, cudaStream_t st) {
+  const Layer &l = n->L[li];
+  switch (l.nc * 1000 + l.cn) {
+    case 16016: return conv_dx_t<2, 16, 2, 27, 1>(n, l, gin, st);
+    case 16032: return conv_dx_t<4, 16, 1, 27, 1>(n, l, gin, st);
+    case 32032: return conv_dx_t<4, 32, 1, 3, 2>(n, l, gin, st);
+    case 32064: return conv_dx_t<8, 32, 1, 3, 2>(n, l, gin, st);
+    case 32128: return conv_dx_t<16, 32, 1, 1, 2>(n, l, gin, st);
+    case 48016: return conv_dx_t<2, 48, 1, 3, 4>(n, l, gin, st);
+  }
+  return set_err(APHID_UNET_ERR_BADARG, "no data-gradient kernel for this layer");
 }
 
 // gOut: gradient of this layer's output (FP32 [Vp][cn]); adds into the input's gradient
@@ -598,11 +609,7 @@ int conv_back(aphid_unet *n, int li, const float *gout, const __nv_bfloat16 *out
   UR(gemm_bf16(n->colT, (int)v.Vp, n->dZT, (int)v.Vp, l.gWT, l.cn, nullptr, l.kp, l.cn, (int)v.Vp, OUT_F32_ATOMIC,
                splitk, st, n->err));
   if (li == 0) return APHID_UNET_OK;  // no gradient for the input features
-  switch (l.nc) {
-    case 16: return conv_dx_t<16, 4>(n, l, n->grad[io], st);
-    case 32: return conv_dx_t<32, 2>(n, l, n->grad[io], st);
-    default: return conv_dx_t<48, 1>(n, l, n->grad[io], st);
-  }
+  return conv_dx(n, li, n->grad[io], st);
 }
 
 int forward(aphid_unet *n, const float *x, cudaStream_t st) {
@@ -729,7 +736,7 @@ int aphid_unet_create(aphid_unet **out, int X, int Y, int Z, int train, unsigned
     Layer l;
     l.cin = kLayerDef[li][0], l.cout = kLayerDef[li][1], l.level = kLayerDef[li][2], l.relu = kLayerDef[li][3];
     l.cg = (int)rup(l.cin, 8), l.cn = (int)rup(l.cout, 16);
-    l.nc = l.cg % 48 == 0 ? 48 : l.cg % 32 == 0 ? 32 : 16;
+    l.nc = l.cg % 32 == 0 ? 32 : l.cg % 48 == 0 ? 48 : 16;
     l.kp = (int)rup(27LL * l.cg, kBM);
     const size_t nw = 27ULL * l.cin * l.cout;
     colmax = std::max(colmax, (size_t)n->vol[l.level].Vp * l.kp);

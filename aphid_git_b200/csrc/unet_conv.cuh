@@ -29,17 +29,12 @@ namespace unet {
 constexpr int kTX = 8, kTY = 16, kRowB = (kTX + 2) * 16, kPlaneB = (kTY + 2) * kRowB;  // tile, bytes of a staged row, plane
 constexpr int kConvThreads = 192;  // warps 0-3: epilogue, 4: producer, 5: MMA issuer
 constexpr int kMaxStages = 4;
+constexpr uint32_t kLast = 2 * (16 + kRowB + kPlaneB);  // the last tap's offset in the staged tile
 
 struct ConvArgs {
-  int X, Y, Z;         // volume
-  long long Vp;        // voxels per plane of 8 channels
-  int ch;              // 8-channel planes of the input
-  int bz;              // z-planes per tile
-  int tx, ty;          // tiles along x, y
-  int chunks;          // K chunks (8 channels of one tap) in the weight stream, even
-  int per_stage;       // chunks per weight stage, even (forward); taps per stage (data gradient)
-  int stages;          // weight stages
-  unsigned chunk_b;    // bytes of a weight chunk: outputs x 16 (forward); of a tap (data gradient)
+  int X, Y, Z;    // volume
+  long long Vp;   // voxels per plane of 8 channels
+  int tx, ty;     // tiles along x, y
 };
 
 // shared-memory descriptor of an unswizzled K-major operand: lbo between the
@@ -57,6 +52,11 @@ __device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.b32 %0, 1, 0, q;\n}\n" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void g_mbar_init_n(uint32_t bar, uint32_t n) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(n) : "memory");
@@ -91,11 +91,11 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // (with one plane of 8 channels the last K = 16 step has no second tap: its
 // operand is a plane of zeros behind the tile, not a neighbour's value times a
 // zero weight, which an infinity would turn into NaN)
-__host__ __device__ constexpr size_t conv_tile_bytes(int ch, int bz) {
-  return ((size_t)(ch * (bz + 2) + (ch & 1)) * kPlaneB + 127) / 128 * 128;
+__host__ __device__ constexpr uint32_t conv_tile_bytes(int ch, int bz) {
+  return ((ch * (bz + 2) + (ch & 1)) * kPlaneB + 127) / 128 * 128;
 }
-inline size_t conv_shm(const ConvArgs &a) {
-  return 128 + conv_tile_bytes(a.ch, a.bz) + (size_t)a.stages * (a.per_stage * a.chunk_b) + 256;
+__host__ __device__ constexpr uint32_t conv_shm(int ch, int bz, uint32_t weight_bytes) {
+  return 128 + conv_tile_bytes(ch, bz) + weight_bytes + 256;
 }
 
 struct ConvShm {
@@ -103,19 +103,21 @@ struct ConvShm {
   uint64_t *full, *empty, *tile_in, *tfull, *tempty;  // [kMaxStages] x 2, 1, 2, 2
   uint32_t *tslot;
 };
-// carve the dynamic shared memory, allocate `cols` of tensor memory, arm the barriers
-__device__ __forceinline__ ConvShm conv_init(unsigned char *raw, const ConvArgs &a, uint32_t cols, uint32_t &tmem) {
+// carve the dynamic shared memory (WB bytes of weight stages), allocate COLS of
+// tensor memory, arm the barriers
+template <int CH, int BZ, uint32_t WB, uint32_t COLS>
+__device__ __forceinline__ ConvShm conv_init(unsigned char *raw, uint32_t &tmem) {
   ConvShm s;
   s.tile = raw + ((128u - (gsm(raw) & 127u)) & 127u);
-  s.w = s.tile + conv_tile_bytes(a.ch, a.bz);
-  s.full = reinterpret_cast<uint64_t *>(s.w + (size_t)a.stages * (a.per_stage * a.chunk_b));
+  s.w = s.tile + conv_tile_bytes(CH, BZ);
+  s.full = reinterpret_cast<uint64_t *>(s.w + WB);
   s.empty = s.full + kMaxStages;
   s.tile_in = s.empty + kMaxStages;
   s.tfull = s.tile_in + 1;
   s.tempty = s.tfull + 2;
   s.tslot = reinterpret_cast<uint32_t *>(s.tempty + 2);
   if (threadIdx.x < 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(gsm(s.tslot)), "r"(cols)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(gsm(s.tslot)), "r"(COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
@@ -132,8 +134,8 @@ __device__ __forceinline__ ConvShm conv_init(unsigned char *raw, const ConvArgs 
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
-  if (a.ch & 1) {
-    uint4 *z = reinterpret_cast<uint4 *>(s.tile + (size_t)a.ch * (a.bz + 2) * kPlaneB);
+  if (CH & 1) {
+    uint4 *z = reinterpret_cast<uint4 *>(s.tile + CH * (BZ + 2) * kPlaneB);
     for (int q = threadIdx.x; q < kPlaneB / 16; q += kConvThreads) z[q] = make_uint4(0, 0, 0, 0);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   }
@@ -151,62 +153,100 @@ __device__ __forceinline__ void conv_exit(uint32_t tmem, uint32_t cols) {
 }
 __host__ __device__ constexpr uint32_t tmem_cols(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512; }
 
-// Forward: out = act(conv(in) + bias), BN output channels, BZ z-planes per
-// block.  Weights: the stream [K chunk][BN][8] (K = tap x channels, in that
-// order), read once per block through a ring.  The products are added in the
-// order of K, 16 at a time.  RELU: BF16 planes of 8 channels; else FP32 rows
-// [Vp][BN] (the head).
-template <int BN, int BZ, bool RELU>
+// offset of the tap after the one at (dx, dy) in the staged tile
+__device__ __forceinline__ void next_tap(uint32_t &at, int &dx, int &dy) {
+  at += 16;
+  if (++dx == 3) {
+    dx = 0, at += kRowB - 48;
+    if (++dy == 3) dy = 0, at += kPlaneB - 3 * kRowB;
+  }
+}
+
+// Forward: out = act(conv(in) + bias) from CH planes of 8 channels to BN output
+// channels, BZ z-planes per block.  Weights: the stream [K chunk][BN][8] (K = tap
+// x channels, in that order), read once per block through a ring of ST stages of
+// PER chunks.  The products are added in the order of K, 16 at a time.  RELU:
+// BF16 planes of 8 channels; else FP32 rows [Vp][BN] (the head).
+// The issuing warp runs its loop as a whole, with every extent a constant, and
+// elects a lane for the instruction alone: one diverged lane with run-time
+// extents spent 160 cycles on the indexes of each K = 16 step and 630 on each
+// weight stage, against the 64 of a 128 x 128 x 16 product.
+template <int CH, int BN, int BZ, int PER, int ST, bool RELU>
 __global__ void __launch_bounds__(kConvThreads) k_conv_fwd(const __grid_constant__ CUtensorMap map, const ConvArgs a,
                                                            const __nv_bfloat16 *__restrict__ wgt,
                                                            const float *__restrict__ bias, void *__restrict__ out, int *err) {
   extern __shared__ unsigned char cs_raw[];
-  constexpr uint32_t kCols = tmem_cols(BN * BZ);
+  static_assert(CH == 1 || CH % 2 == 0, "K = 16: two planes of a tap, or two taps of one plane");
+  static_assert(PER % 2 == 0 && ST <= kMaxStages, "weight stages");
+  constexpr int kChunks = (27 * CH + 1) / 2 * 2, kStages = (kChunks + PER - 1) / PER;
+  constexpr uint32_t kCols = tmem_cols(BN * BZ), chunk_b = BN * 16, stage_b = PER * chunk_b, plane_b = (BZ + 2) * kPlaneB;
   uint32_t tmem;
-  const ConvShm s = conv_init(cs_raw, a, kCols, tmem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const ConvShm s = conv_init<CH, BZ, ST * stage_b, kCols>(cs_raw, tmem);
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   int b = blockIdx.x;
   const int x0 = b % a.tx * kTX;
   b /= a.tx;
   const int y0 = b % a.ty * kTY, z0 = b / a.ty * BZ;
-  const int nst = (a.chunks + a.per_stage - 1) / a.per_stage;
-  const uint32_t stage_b = a.per_stage * a.chunk_b, plane_b = (BZ + 2) * kPlaneB;
   bool ok = true;
-  if (warp == 4 && lane == 0) {
-    g_mbar_expect(gsm(s.tile_in), (uint32_t)a.ch * plane_b);
-    g_tma_load4(gsm(s.tile), &map, (x0 - 1) * 8, y0 - 1, z0 - 1, 0, gsm(s.tile_in));
-    for (int q = 0; q < nst; q++) {
-      const int st = q % a.stages;
-      if (q >= a.stages && ok) ok = g_mbar_wait(gsm(&s.empty[st]), (uint32_t)((q / a.stages - 1) & 1));
-      const uint32_t bytes = min(a.per_stage, a.chunks - q * a.per_stage) * a.chunk_b;
-      g_mbar_expect(gsm(&s.full[st]), bytes);
-      g_bulk_load(gsm(s.w) + st * stage_b, wgt + (size_t)q * stage_b / 2, bytes, gsm(&s.full[st]));
+  if (warp == 4) {
+    if (lane == 0) {
+      g_mbar_expect(gsm(s.tile_in), CH * plane_b);
+      g_tma_load4(gsm(s.tile), &map, (x0 - 1) * 8, y0 - 1, z0 - 1, 0, gsm(s.tile_in));
+      int st = 0, lap = 0;
+      for (int q = 0; q < kStages; q++) {
+        if (lap > 0 && ok) ok = g_mbar_wait(gsm(&s.empty[st]), (uint32_t)((lap - 1) & 1));
+        const uint32_t bytes = min(PER, kChunks - q * PER) * chunk_b;
+        g_mbar_expect(gsm(&s.full[st]), bytes);
+        g_bulk_load(gsm(s.w) + st * stage_b, wgt + (size_t)q * stage_b / 2, bytes, gsm(&s.full[st]));
+        if (++st == ST) st = 0, lap++;
+      }
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == 5) {
     constexpr uint32_t idesc = idesc_bf16(kBM, BN);
+    const bool lead = elect_one();
     ok = g_mbar_wait(gsm(s.tile_in), 0u);
-    const uint32_t tile = gsm(s.tile);
-    auto tap_at = [](int t) { return (uint32_t)(t % 3 * 16 + t / 3 % 3 * kRowB + t / 9 * kPlaneB); };
-    for (int q = 0; q < nst; q++) {
-      const int st = q % a.stages;
-      if (ok) ok = g_mbar_wait(gsm(&s.full[st]), (uint32_t)((q / a.stages) & 1));
+    const uint64_t da0 = smem_desc(gsm(s.tile), plane_b, kRowB), db0 = smem_desc(gsm(s.w), chunk_b, 128);
+    uint32_t at = 0, c_at = 0;  // tap, channel plane: bytes from the tile's start
+    int dx = 0, dy = 0, st = 0, lap = 0;
+#pragma unroll 1
+    for (int q = 0; q < kStages; q++) {
+      if (ok) ok = g_mbar_wait(gsm(&s.full[st]), (uint32_t)(lap & 1));
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const int k1 = min(a.chunks, (q + 1) * a.per_stage);
-      for (int k = q * a.per_stage; k < k1; k += 2) {
-        const int t = k / a.ch, c = k - t * a.ch;
-        // K = 16: two planes of one tap, or (one plane) two taps, the last with zeros
-        const uint32_t at = tap_at(t);
-        const uint64_t db = smem_desc(gsm(s.w) + st * stage_b + (k - q * a.per_stage) * a.chunk_b, a.chunk_b, 128);
-        const uint32_t a0 = tile + c * plane_b + at;
+      const int steps = min(PER, kChunks - q * PER) / 2;
+      uint64_t db = db0 + (uint64_t)((uint32_t)st * stage_b >> 4);
+#pragma unroll(PER <= 16 ? PER / 2 : 4)
+      for (int k = 0; k < steps; k++) {
+        const uint32_t acc = q > 0 || k > 0;
+        uint64_t da = da0 + (uint64_t)((at + c_at) >> 4);
+        uint32_t lbo = plane_b;  // two planes of one tap
+        if (CH == 1) {           // two taps, the last with zeros
+          const uint32_t t0 = at;
+          next_tap(at, dx, dy);
+          lbo = at - t0;
+          da = smem_desc(gsm(s.tile) + t0, lbo, kRowB);
+          if (q * PER / 2 + k == kChunks / 2 - 1) lbo = 0;
+        }
+        if (lead) {
 #pragma unroll
-        for (int p = 0; p < BZ; p++) {
-          const uint32_t lbo = a.ch > 1 ? plane_b : t < 26 ? tap_at(t + 1) - at : plane_b - at - p * kPlaneB;
-          mma_f16(tmem + p * BN, smem_desc(a0 + p * kPlaneB, lbo, kRowB), db, idesc, k > 0);
+          for (int p = 0; p < BZ; p++) {
+            if (CH == 1 && lbo == 0)
+              mma_f16(tmem + p * BN, smem_desc(gsm(s.tile) + kLast + p * kPlaneB, plane_b - kLast - p * kPlaneB, kRowB), db, idesc, acc);
+            else
+              mma_f16(tmem + p * BN, da + p * (kPlaneB >> 4), db, idesc, acc);
+          }
+        }
+        db += 2 * chunk_b >> 4;
+        if (CH == 1) {
+          next_tap(at, dx, dy);
+        } else if ((c_at += 2 * plane_b) == CH * plane_b) {
+          c_at = 0;
+          next_tap(at, dx, dy);
         }
       }
-      mma_commit(gsm(&s.empty[st]));
+      if (lead) mma_commit(gsm(&s.empty[st]));
+      if (++st == ST) st = 0, lap++;
     }
-    mma_commit(gsm(s.tfull));
+    if (lead) mma_commit(gsm(s.tfull));
   }
   __syncwarp();
   if (warp < 4) {
@@ -221,7 +261,7 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_fwd(const __grid_constant
       const int z = z0 + p;
       const long long v = x + (long long)a.X * (y + (long long)a.Y * z);
       const bool in = x < a.X && y < a.Y && z < a.Z;
-#pragma unroll
+#pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 16) {
         float f[16];
         __syncwarp();
@@ -253,62 +293,73 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_fwd(const __grid_constant
 }
 
 // Data gradient: gin[u][c] += sum over the taps t = 0 .. 26 of
-// sum_co dz[u - d_t][co] W[co][t][c], NC input channels of group blockIdx.y, BZ
-// z-planes per block.  Each tap's products are formed in tensor memory on their
-// own and added in FP32 registers in the order of the taps, as a column matrix
-// and its gather would add them: a sum over the taps inside tensor memory would
-// round differently, and the next layer's BF16 rounding turns that into steps.
-// Two tensor-memory buffers: the tap after the one being added is in flight.
-// Weights: [group][tap][co / 8][NC][8].
-template <int NC, int BZ>
+// sum_co dz[u - d_t][co] W[co][t][c], NC input channels of group blockIdx.y, CH
+// planes of dz, BZ z-planes per block.  Each tap's products are formed in tensor
+// memory on their own and added in FP32 registers in the order of the taps, as a
+// column matrix and its gather would add them: a sum over the taps inside tensor
+// memory would round differently, and the next layer's BF16 rounding turns that
+// into steps.  Two tensor-memory buffers: the tap after the one being added is in
+// flight.  Weights: [group][tap][co / 8][NC][8], ST stages of PER taps.
+template <int CH, int NC, int BZ, int PER, int ST>
 __global__ void __launch_bounds__(kConvThreads) k_conv_dx(const __grid_constant__ CUtensorMap map, const ConvArgs a,
                                                           const __nv_bfloat16 *__restrict__ wgt, int C,
                                                           float *__restrict__ gin, int *err) {
   extern __shared__ unsigned char cs_raw[];
-  constexpr uint32_t kCols = tmem_cols(2 * NC * BZ);
+  static_assert(CH % 2 == 0 && ST <= kMaxStages, "K = 16, weight stages");
+  constexpr int kTaps = 27, kStages = (kTaps + PER - 1) / PER;
+  constexpr uint32_t kCols = tmem_cols(2 * NC * BZ), tap_b = CH * NC * 16, stage_b = PER * tap_b, plane_b = (BZ + 2) * kPlaneB;
   uint32_t tmem;
-  const ConvShm s = conv_init(cs_raw, a, kCols, tmem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const ConvShm s = conv_init<CH, BZ, ST * stage_b, kCols>(cs_raw, tmem);
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   int b = blockIdx.x;
   const int x0 = b % a.tx * kTX;
   b /= a.tx;
   const int y0 = b % a.ty * kTY, z0 = b / a.ty * BZ;
-  constexpr int kTaps = 27;
-  const int nst = (kTaps + a.per_stage - 1) / a.per_stage;
-  const uint32_t stage_b = a.per_stage * a.chunk_b, plane_b = (BZ + 2) * kPlaneB;
   bool ok = true;
-  if (warp == 4 && lane == 0) {
-    const __nv_bfloat16 *w = wgt + (size_t)blockIdx.y * kTaps * a.chunk_b / 2;
-    g_mbar_expect(gsm(s.tile_in), (uint32_t)a.ch * plane_b);
-    g_tma_load4(gsm(s.tile), &map, (x0 - 1) * 8, y0 - 1, z0 - 1, 0, gsm(s.tile_in));
-    for (int q = 0; q < nst; q++) {
-      const int st = q % a.stages;
-      if (q >= a.stages && ok) ok = g_mbar_wait(gsm(&s.empty[st]), (uint32_t)((q / a.stages - 1) & 1));
-      const uint32_t bytes = min(a.per_stage, kTaps - q * a.per_stage) * a.chunk_b;
-      g_mbar_expect(gsm(&s.full[st]), bytes);
-      g_bulk_load(gsm(s.w) + st * stage_b, w + (size_t)q * stage_b / 2, bytes, gsm(&s.full[st]));
+  if (warp == 4) {
+    if (lane == 0) {
+      const __nv_bfloat16 *w = wgt + (size_t)blockIdx.y * kTaps * tap_b / 2;
+      g_mbar_expect(gsm(s.tile_in), CH * plane_b);
+      g_tma_load4(gsm(s.tile), &map, (x0 - 1) * 8, y0 - 1, z0 - 1, 0, gsm(s.tile_in));
+      int st = 0, lap = 0;
+      for (int q = 0; q < kStages; q++) {
+        if (lap > 0 && ok) ok = g_mbar_wait(gsm(&s.empty[st]), (uint32_t)((lap - 1) & 1));
+        const uint32_t bytes = min(PER, kTaps - q * PER) * tap_b;
+        g_mbar_expect(gsm(&s.full[st]), bytes);
+        g_bulk_load(gsm(s.w) + st * stage_b, w + (size_t)q * stage_b / 2, bytes, gsm(&s.full[st]));
+        if (++st == ST) st = 0, lap++;
+      }
     }
-  } else if (warp == 5 && lane == 0) {
+  } else if (warp == 5) {
     constexpr uint32_t idesc = idesc_bf16(kBM, NC);
+    const bool lead = elect_one();
     ok = g_mbar_wait(gsm(s.tile_in), 0u);
-    const uint32_t tile = gsm(s.tile);
+    const uint64_t da0 = smem_desc(gsm(s.tile), plane_b, kRowB), db0 = smem_desc(gsm(s.w), NC * 16, 128);
+    uint32_t at = 0;
+    int dx = 0, dy = 0, st = 0, lap = 0, left = PER;
+#pragma unroll 1
     for (int t = 0; t < kTaps; t++) {
-      const int q = t / a.per_stage, st = q % a.stages, buf = t & 1;
-      if (t == q * a.per_stage && ok) ok = g_mbar_wait(gsm(&s.full[st]), (uint32_t)((q / a.stages) & 1));
+      const int buf = t & 1;
+      if (left == PER && ok) ok = g_mbar_wait(gsm(&s.full[st]), (uint32_t)(lap & 1));
       if (t >= 2 && ok) ok = g_mbar_wait(gsm(&s.tempty[buf]), (uint32_t)((t / 2 - 1) & 1));
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       // u - d_t: the staged voxel 1 - d_t on
-      const uint32_t at = (uint32_t)((2 - t % 3) * 16 + (2 - t / 3 % 3) * kRowB + (2 - t / 9) * kPlaneB);
-      const uint32_t w0 = gsm(s.w) + st * stage_b + (t - q * a.per_stage) * a.chunk_b;
-      for (int c = 0; c < a.ch; c += 2) {
-        const uint64_t db = smem_desc(w0 + c * (NC * 16), NC * 16, 128);
-        const uint32_t a0 = tile + c * plane_b + at;
+      const uint64_t da = da0 + (uint64_t)((kLast - at) >> 4);
+      const uint64_t db = db0 + (uint64_t)(((uint32_t)st * stage_b + (uint32_t)(PER - left) * tap_b) >> 4);
+      if (lead) {
 #pragma unroll
-        for (int p = 0; p < BZ; p++)
-          mma_f16(tmem + (buf * BZ + p) * NC, smem_desc(a0 + p * kPlaneB, plane_b, kRowB), db, idesc, c > 0);
+        for (int c = 0; c < CH; c += 2)
+#pragma unroll
+          for (int p = 0; p < BZ; p++)
+            mma_f16(tmem + (buf * BZ + p) * NC, da + ((c * plane_b + p * kPlaneB) >> 4), db + (c * NC), idesc, c > 0);
+        mma_commit(gsm(&s.tfull[buf]));
       }
-      mma_commit(gsm(&s.tfull[buf]));
-      if (t + 1 == kTaps || (t + 1) % a.per_stage == 0) mma_commit(gsm(&s.empty[st]));
+      next_tap(at, dx, dy);
+      if (--left == 0 || t + 1 == kTaps) {
+        if (lead) mma_commit(gsm(&s.empty[st]));
+        left = PER;
+        if (++st == ST) st = 0, lap++;
+      }
     }
   }
   __syncwarp();
