@@ -1,7 +1,6 @@
 // aphid_unet.cu -- the initial-guess network's device side: the tcgen05 BF16
 // GEMM launcher and (below) the layers: convolutions as implicit GEMMs
-// (unet_conv.cuh), the weight gradient as a split-K GEMM over a transposed column
-// matrix, and the memory-bound passes between them.  Activations are BF16 in
+// (unet_conv.cuh) and the memory-bound passes between them.  Activations are BF16 in
 // planes of 8 channels [C/8][Vp][8], gradients FP32 channels last [Vp][C].
 // C ABI in include/aphid_unet.h.
 #include <cuda_bf16.h>
@@ -135,91 +134,60 @@ struct Vol {
 
 // ---------------------------------------------------------------- kernels
 // features [V][3] (original volume) -> [Vp][8] BF16 on the padded volume
+// (a voxel index fits 32 bits: 2^32 voxels would be 400 GB of activations; a
+// 64-bit division per value made these passes 2 to 8 x their memory time)
+struct Xyz { int x, y, z; };
+__device__ __forceinline__ Xyz xyz(unsigned r, int X, int Y) {
+  const unsigned q = r / (unsigned)X, z = q / (unsigned)Y;
+  return {(int)(r - q * X), (int)(q - z * Y), (int)z};
+}
 __global__ void k_pack_in(const float *__restrict__ x, int X, int Y, int Z, Vol v, __nv_bfloat16 *__restrict__ a) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < v.Vp * 8; t += (long long)gridDim.x * blockDim.x) {
-    const long long r = t >> 3;
-    const int c = (int)(t & 7);
-    float val = 0.f;
-    if (r < v.V && c < 3) {
-      const int px = (int)(r % v.X), py = (int)((r / v.X) % v.Y), pz = (int)(r / ((long long)v.X * v.Y));
-      if (px < X && py < Y && pz < Z) val = x[(px + (long long)X * (py + (long long)Y * pz)) * 3 + c];
+  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < v.Vp; r += (long long)gridDim.x * blockDim.x) {
+    float f[3] = {};
+    if (r < v.V) {
+      const Xyz p = xyz((unsigned)r, v.X, v.Y);
+      if (p.x < X && p.y < Y && p.z < Z) {
+        const float *s = x + (p.x + (long long)X * (p.y + (long long)Y * p.z)) * 3;
+        f[0] = s[0], f[1] = s[1], f[2] = s[2];
+      }
     }
-    a[t] = __float2bfloat16_rn(val);
+    auto b = [](float q) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(q)); };
+    reinterpret_cast<uint4 *>(a)[r] = make_uint4(b(f[0]) | (b(f[1]) << 16), b(f[2]), 0, 0);
   }
 }
 // head output [Vp][16] FP32 -> [V][8] on the original volume
 __global__ void k_unpack_out(const float *__restrict__ y, int X, int Y, int Z, Vol v, float *__restrict__ o) {
-  const long long n = (long long)X * Y * Z * 8;
+  const long long n = (long long)X * Y * Z * 2;
+  const bool vec = ((uintptr_t)o & 15) == 0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const long long r = t >> 3;
-    const int c = (int)(t & 7);
-    const int px = (int)(r % X), py = (int)((r / X) % Y), pz = (int)(r / ((long long)X * Y));
-    o[t] = y[(px + (long long)v.X * (py + (long long)v.Y * pz)) * 16 + c];
+    const Xyz p = xyz((unsigned)(t >> 1), X, Y);
+    const float4 f = reinterpret_cast<const float4 *>(y)[(p.x + (long long)v.X * (p.y + (long long)v.Y * p.z)) * 4 + (t & 1)];
+    if (vec)
+      reinterpret_cast<float4 *>(o)[t] = f;
+    else
+      o[4 * t] = f.x, o[4 * t + 1] = f.y, o[4 * t + 2] = f.z, o[4 * t + 3] = f.w;
   }
 }
 
-// colT [kp][Vp], the transposed column matrix of the weight gradient:
-// colT[t*C + c][r] = in[r + d_t][c] (zero outside, pads zero), in in planes of 8
-// channels.  A thread turns 8 voxels x 8 channels around in registers: 16-byte
-// loads and stores (single values cost 99 us a layer of the 72 x 72 x 56
-// training volume on average).
-__global__ void k_im2colT(const __nv_bfloat16 *__restrict__ in, int C, Vol v, int kp, __nv_bfloat16 *__restrict__ colT) {
-  const int kc = kp / 8, used = 27 * C / 8;
-  const long long groups = v.Vp / 8;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < groups * kc; t += (long long)gridDim.x * blockDim.x) {
-    const int q = (int)(t / groups);
-    const long long r0 = (t - q * groups) * 8;
-    uint4 val[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) val[j] = make_uint4(0, 0, 0, 0);
-    if (q < used) {
-      const int tap = q / (C / 8), c8 = q % (C / 8);
-      const uint4 *src = reinterpret_cast<const uint4 *>(in) + c8 * v.Vp;
-      const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-      int x = (int)(r0 % v.X), y = (int)((r0 / v.X) % v.Y), z = (int)(r0 / ((long long)v.X * v.Y));
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int nx = x + dx, ny = y + dy, nz = z + dz;
-        if (z < v.Z && nx >= 0 && ny >= 0 && nz >= 0 && nx < v.X && ny < v.Y && nz < v.Z)
-          val[j] = src[nx + (long long)v.X * (ny + (long long)v.Y * nz)];
-        if (++x == v.X) {
-          x = 0;
-          if (++y == v.Y) y = 0, z++;
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 8; c++) {  // channel c of the 8 voxels
-      uint32_t o[4];
-#pragma unroll
-      for (int h = 0; h < 4; h++) {
-        auto word = [&](const uint4 &w) { return c < 2 ? w.x : c < 4 ? w.y : c < 6 ? w.z : w.w; };
-        o[h] = __byte_perm(word(val[2 * h]), word(val[2 * h + 1]), c & 1 ? 0x7632 : 0x5410);
-      }
-      *reinterpret_cast<uint4 *>(colT + (long long)(q * 8 + c) * v.Vp + r0) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-  }
-}
-// a value of an activation in planes of 8 channels
-__device__ __forceinline__ float act_at(const __nv_bfloat16 *act, const Vol &v, long long r, int c) {
-  return __bfloat162float(act[((c >> 3) * v.Vp + r) * 8 + (c & 7)]);
-}
-// dz = g * (act > 0) (relu) or g; dZ in planes of 8 channels and dZT [cn][Vp],
-// both BF16, rows past the volume zero.  A thread takes 8 channels of a voxel.
+// dz = g * (act > 0) (relu) or g; dZ in planes of 8 channels, BF16, rows past the
+// volume zero, and gb[c] += sum_r dz[r][c] before the rounding.  A thread takes 8
+// channels (plane blockIdx.y) of its voxels; gb has room for whole planes.
 __global__ void k_relu_back(const float *__restrict__ g, const __nv_bfloat16 *__restrict__ act, int C, int relu, Vol v,
-                            __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *__restrict__ dZT) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < v.Vp * (C / 8); t += (long long)gridDim.x * blockDim.x) {
-    const int c8 = (int)(t / v.Vp);
-    const long long r = t - c8 * v.Vp;
+                            __nv_bfloat16 *__restrict__ dZ, float *__restrict__ gb) {
+  const int c8 = blockIdx.y;
+  float sum[8] = {};
+  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < v.Vp; r += (long long)gridDim.x * blockDim.x) {
     float d[8] = {};
     if (r < v.V) {
       const float4 *s = reinterpret_cast<const float4 *>(g + r * C + c8 * 8);
       const float4 a = s[0], b = s[1];
       d[0] = a.x, d[1] = a.y, d[2] = a.z, d[3] = a.w, d[4] = b.x, d[5] = b.y, d[6] = b.z, d[7] = b.w;
       if (relu) {
+        const uint4 w = reinterpret_cast<const uint4 *>(act)[c8 * v.Vp + r];
+        const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&w);
 #pragma unroll
         for (int j = 0; j < 8; j++)
-          if (!(act_at(act, v, r, c8 * 8 + j) > 0.f)) d[j] = 0.f;
+          if (!(__bfloat162float(e[j]) > 0.f)) d[j] = 0.f;
       }
     }
     uint32_t o[4];
@@ -227,55 +195,42 @@ __global__ void k_relu_back(const float *__restrict__ g, const __nv_bfloat16 *__
     for (int j = 0; j < 4; j++)
       o[j] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(d[2 * j])) |
              ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(d[2 * j + 1])) << 16);
-    reinterpret_cast<uint4 *>(dZ)[t] = make_uint4(o[0], o[1], o[2], o[3]);
+    reinterpret_cast<uint4 *>(dZ)[c8 * v.Vp + r] = make_uint4(o[0], o[1], o[2], o[3]);
 #pragma unroll
-    for (int j = 0; j < 8; j++) dZT[(long long)(c8 * 8 + j) * v.Vp + r] = __ushort_as_bfloat16((unsigned short)(o[j / 2] >> (16 * (j & 1))));
+    for (int j = 0; j < 8; j++) sum[j] += d[j];
   }
-}
-// gb[c] += sum_r dz[r][c] (FP32 dz, before rounding)
-__global__ void k_bias_grad(const float *__restrict__ g, const __nv_bfloat16 *__restrict__ act, int C, int relu, Vol v,
-                            float *__restrict__ gb) {
-  const int c = blockIdx.y;
-  float s = 0.f;
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < v.V; r += (long long)gridDim.x * blockDim.x) {
-    float d = g[r * C + c];
-    if (relu && !(act_at(act, v, r, c) > 0.f)) d = 0.f;
-    s += d;
+  __shared__ float sh[kT / 32][8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    for (int o = 16; o; o >>= 1) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][j] = sum[j];
   }
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ float sh[kT / 32];
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 8) {
     float t = 0.f;
-    for (int q = 0; q < kT / 32; q++) t += sh[q];
-    atomicAdd(gb + c, t);
+    for (int q = 0; q < kT / 32; q++) t += sh[q][threadIdx.x];
+    atomicAdd(gb + c8 * 8 + threadIdx.x, t);
   }
 }
-// 2x2x2 mean: fine volume f -> coarse volume o, in planes of 8 channels
-__global__ void k_pool(const __nv_bfloat16 *__restrict__ in, int C, Vol f, Vol o, __nv_bfloat16 *__restrict__ out) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < o.Vp * (C / 8); t += (long long)gridDim.x * blockDim.x) {
-    const int c8 = (int)(t / o.Vp);
-    const long long r = t - c8 * o.Vp;
+// 2x2x2 mean: fine volume f -> coarse volume o, plane blockIdx.y of 8 channels
+__global__ void k_pool(const __nv_bfloat16 *__restrict__ in, Vol f, Vol o, __nv_bfloat16 *__restrict__ out) {
+  const int c8 = blockIdx.y;
+  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < o.V; r += (long long)gridDim.x * blockDim.x) {
+    const Xyz p = xyz((unsigned)r, o.X, o.Y);
     float s[8] = {};
-    if (r < o.V) {
-      const int x = (int)(r % o.X), y = (int)((r / o.X) % o.Y), z = (int)(r / ((long long)o.X * o.Y));
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const long long fr = (2 * x + (q & 1)) + (long long)f.X * ((2 * y + ((q >> 1) & 1)) + (long long)f.Y * (2 * z + (q >> 2)));
-        const uint4 w = reinterpret_cast<const uint4 *>(in)[c8 * f.Vp + fr];
-        const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&w);
+    for (int q = 0; q < 8; q++) {
+      const long long fr = (2 * p.x + (q & 1)) + (long long)f.X * ((2 * p.y + ((q >> 1) & 1)) + (long long)f.Y * (2 * p.z + (q >> 2)));
+      const uint4 w = reinterpret_cast<const uint4 *>(in)[c8 * f.Vp + fr];
+      const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&w);
 #pragma unroll
-        for (int c = 0; c < 8; c++) s[c] += __bfloat162float(e[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < 8; c++) s[c] *= 0.125f;
+      for (int c = 0; c < 8; c++) s[c] += __bfloat162float(e[c]);
     }
     uint4 w;
     __nv_bfloat16 *e = reinterpret_cast<__nv_bfloat16 *>(&w);
 #pragma unroll
-    for (int c = 0; c < 8; c++) e[c] = __float2bfloat16_rn(s[c]);
-    reinterpret_cast<uint4 *>(out)[t] = w;
+    for (int c = 0; c < 8; c++) e[c] = __float2bfloat16_rn(s[c] * 0.125f);
+    reinterpret_cast<uint4 *>(out)[c8 * o.Vp + r] = w;
   }
 }
 // gf[child][c] += go[parent][c] / 8
@@ -287,26 +242,18 @@ __global__ void k_pool_back(const float *__restrict__ go, int C, Vol f, Vol o, f
     gf[t] += 0.125f * go[((x >> 1) + (long long)o.X * ((y >> 1) + (long long)o.Y * (z >> 1))) * C + c];
   }
 }
-// cat[r] = up(low)[r] (Cu channels) ++ skip[r] (Cs channels) on the fine volume,
-// in planes of 8 channels
-__global__ void k_upcat(const __nv_bfloat16 *__restrict__ low, int Cu, const __nv_bfloat16 *__restrict__ skip, int Cs,
-                        Vol f, Vol o, __nv_bfloat16 *__restrict__ cat) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < f.Vp * ((Cu + Cs) / 8); t += (long long)gridDim.x * blockDim.x) {
-    const int c8 = (int)(t / f.Vp);
-    const long long r = t - c8 * f.Vp;
-    uint4 val = make_uint4(0, 0, 0, 0);
-    if (r < f.V) {
-      if (c8 < Cu / 8) {
-        const int x = (int)(r % f.X), y = (int)((r / f.X) % f.Y), z = (int)(r / ((long long)f.X * f.Y));
-        val = reinterpret_cast<const uint4 *>(low)[c8 * o.Vp + (x >> 1) + (long long)o.X * ((y >> 1) + (long long)o.Y * (z >> 1))];
-      } else {
-        val = reinterpret_cast<const uint4 *>(skip)[(c8 - Cu / 8) * f.Vp + r];
-      }
-    }
-    reinterpret_cast<uint4 *>(cat)[t] = val;
+// the upper half of a concatenation, cat[r] = up(low)[r], plane blockIdx.y of 8
+// channels (the skip's planes follow in the same array and are written there by
+// the layer that computes them)
+__global__ void k_up(const __nv_bfloat16 *__restrict__ low, Vol f, Vol o, __nv_bfloat16 *__restrict__ cat) {
+  const int c8 = blockIdx.y;
+  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < f.V; r += (long long)gridDim.x * blockDim.x) {
+    const Xyz p = xyz((unsigned)r, f.X, f.Y);
+    reinterpret_cast<uint4 *>(cat)[c8 * f.Vp + r] =
+        reinterpret_cast<const uint4 *>(low)[c8 * o.Vp + (p.x >> 1) + (long long)o.X * ((p.y >> 1) + (long long)o.Y * (p.z >> 1))];
   }
 }
-// the gradient of k_upcat: glow[p][c] += sum over the 8 children, gskip += tail
+// the gradient of the concatenation: glow[p][c] += sum over the 8 children, gskip += tail
 __global__ void k_upcat_back_low(const float *__restrict__ gcat, int Cu, int Cs, Vol f, Vol o, float *__restrict__ glow) {
   const int C = Cu + Cs;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < o.V * Cu; t += (long long)gridDim.x * blockDim.x) {
@@ -392,7 +339,7 @@ __global__ void k_cast_w(const float *__restrict__ W, int cin, int cg, int cout,
     if (nc && tap < 27) Wd[((((long long)(ci / nc) * 27 + tap) * (cn / 8) + co / 8) * nc + ci % nc) * 8 + co % 8] = b;
   }
 }
-// Adam on one layer (FP32 master weights), gradient of W from gWT [kp][cn]
+// Adam on one layer (FP32 master weights), gradient of W from gWT [27 cg][cn]
 __global__ void k_adam(float *__restrict__ W, float *__restrict__ m, float *__restrict__ v2, const float *__restrict__ gWT,
                        int cin, int cg, int cout, int cn, float *__restrict__ b, float *__restrict__ mb,
                        float *__restrict__ vb, const float *__restrict__ gb, float lr, float c1, float c2) {
@@ -433,7 +380,7 @@ __global__ void k_grad_out(const float *__restrict__ gWT, const float *__restric
 
 // ----------------------------------------------------------------- network
 struct Layer {
-  int cin, cg, cout, cn, nc, kp, level, relu;  // cg: cin rounded to 8; cn: cout rounded to 16; nc: see k_conv_dx
+  int cin, cg, cout, cn, nc, level, relu;  // cg: cin rounded to 8; cn: cout rounded to 16; nc: see k_conv_dx
   float *W = nullptr, *b = nullptr, *mW = nullptr, *vW = nullptr, *mb = nullptr, *vb = nullptr;
   float *gWT = nullptr, *gb = nullptr;
   __nv_bfloat16 *Wf = nullptr, *Wd = nullptr;
@@ -456,7 +403,9 @@ struct aphid_unet {
   float *grad[aphid::unet::A_COUNT] = {};
   int ach[aphid::unet::A_COUNT], alev[aphid::unet::A_COUNT];
   float *y = nullptr, *gy = nullptr;               // head output / its gradient [Vp][16]
-  __nv_bfloat16 *colT = nullptr, *dZ = nullptr, *dZT = nullptr;
+  __nv_bfloat16 *dZ = nullptr;
+  float *grad_all = nullptr, *gout = nullptr;  // all gradients (zeroed in one pass); the copy in the parameter layout
+  size_t grad_bytes = 0, nparam = 0;
   double *sums = nullptr;
   int *err = nullptr;
   long long step = 0;
@@ -508,12 +457,12 @@ int cast_weights(aphid_unet *n, cudaStream_t st) {
   return APHID_UNET_OK;
 }
 
-// an activation (or dZ) of C channels in planes of 8 as the tensor whose box is
-// a convolution tile of bz z-planes with its halo
-int act_map(CUtensorMap *m, const __nv_bfloat16 *base, int C, const Vol &v, int bz) {
+// an activation (or dZ) of C channels in planes of 8 as a tensor with boxes of
+// bx x by x bz voxels of bc planes
+int act_map(CUtensorMap *m, const __nv_bfloat16 *base, int C, const Vol &v, int bx, int by, int bz, int bc) {
   const cuuint64_t dims[4] = {8 * (cuuint64_t)v.X, (cuuint64_t)v.Y, (cuuint64_t)v.Z, (cuuint64_t)(C / 8)};
   const cuuint64_t strides[3] = {16 * (cuuint64_t)v.X, 16 * (cuuint64_t)v.X * v.Y, 16 * (cuuint64_t)v.Vp};
-  const cuuint32_t box[4] = {8 * (kTX + 2), kTY + 2, (cuuint32_t)(bz + 2), (cuuint32_t)(C / 8)}, es[4] = {1, 1, 1, 1};
+  const cuuint32_t box[4] = {(cuuint32_t)(8 * bx), (cuuint32_t)by, (cuuint32_t)bz, (cuuint32_t)bc}, es[4] = {1, 1, 1, 1};
   EncodeTiledFn fn = encode_fn();
   if (!fn) return set_err(APHID_UNET_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
   const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16 *>(base), dims, strides, box, es,
@@ -527,7 +476,7 @@ int launch_conv(Kernel kernel, const __nv_bfloat16 *in, int C, const Vol &v, int
                 Args... args) {
   ConvArgs a{v.X, v.Y, v.Z, v.Vp, (v.X + kTX - 1) / kTX, (v.Y + kTY - 1) / kTY};
   CUtensorMap m;
-  UR(act_map(&m, in, C, v, bz));
+  UR(act_map(&m, in, C, v, kTX + 2, kTY + 2, bz + 2, C / 8));
   UK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
   kernel<<<dim3((unsigned)(a.tx * a.ty * ((v.Z + bz - 1) / bz)), (unsigned)groups), kConvThreads, shm, st>>>(m, a, args...);
   UK(cudaGetLastError());
@@ -593,35 +542,64 @@ int conv_dx(aphid_unet *n, int li, float *gin, cudaStream_t st) {
   return set_err(APHID_UNET_ERR_BADARG, "no data-gradient kernel for this layer");
 }
 
+template <int CH, int CN>
+int conv_dw_t(aphid_unet *n, const Layer &l, const __nv_bfloat16 *in, cudaStream_t st) {
+  using D = DwShape<CH, CN>;
+  const Vol &v = n->vol[l.level];
+  const ConvArgs a{v.X, v.Y, v.Z, v.Vp, (v.X + kTX - 1) / kTX, (v.Y + kTY - 1) / kTY};
+  CUtensorMap mi, mz;
+  UR(act_map(&mi, in, l.cg, v, kTX + 2, kTY, 1, 1));
+  UR(act_map(&mz, n->dZ, l.cn, v, kTX, kTY, 1, 1));
+  UK(cudaFuncSetAttribute(k_conv_dw<CH, CN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)D::shm));
+  const int tiles = a.tx * a.ty * v.Z;
+  // one wave: two blocks per SM up to 32 outputs, else one
+  const int split = std::max(1, std::min(tiles, (CN <= 32 ? 296 : 148) / D::kGroups));
+  k_conv_dw<CH, CN><<<dim3(D::kGroups, (unsigned)split), kConvThreads, D::shm, st>>>(mi, mz, a, tiles, l.gWT, n->err);
+  UK(cudaGetLastError());
+  return APHID_UNET_OK;
+}
+// The weight gradient of one layer into gWT (zeroed).
+int conv_dw(aphid_unet *n, int li, cudaStream_t st) {
+  const Layer &l = n->L[li];
+  const __nv_bfloat16 *in = n->act[kLayerIO[li][0]];
+  switch (l.cg * 1000 + l.cn) {
+    case 8016: return conv_dw_t<1, 16>(n, l, in, st);
+    case 16016: return conv_dw_t<2, 16>(n, l, in, st);
+    case 16032: return conv_dw_t<2, 32>(n, l, in, st);
+    case 32032: return conv_dw_t<4, 32>(n, l, in, st);
+    case 32064: return conv_dw_t<4, 64>(n, l, in, st);
+    case 64064: return conv_dw_t<8, 64>(n, l, in, st);
+    case 64128: return conv_dw_t<8, 128>(n, l, in, st);
+    case 128128: return conv_dw_t<16, 128>(n, l, in, st);
+    case 192064: return conv_dw_t<24, 64>(n, l, in, st);
+    case 96032: return conv_dw_t<12, 32>(n, l, in, st);
+    case 48016: return conv_dw_t<6, 16>(n, l, in, st);
+  }
+  return set_err(APHID_UNET_ERR_BADARG, "no weight-gradient kernel for this layer");
+}
+
 // gOut: gradient of this layer's output (FP32 [Vp][cn]); adds into the input's gradient
 int conv_back(aphid_unet *n, int li, const float *gout, const __nv_bfloat16 *out, cudaStream_t st) {
   const Layer &l = n->L[li];
   const Vol &v = n->vol[l.level];
   const int io = kLayerIO[li][0];
-  k_relu_back<<<nblk(v.Vp * (l.cn / 8)), kT, 0, st>>>(gout, out, l.cn, l.relu, v, n->dZ, n->dZT);
-  k_bias_grad<<<dim3((unsigned)std::min<long long>((v.V + kT - 1) / kT, 64), (unsigned)l.cout), kT, 0, st>>>(
-      gout, out, l.cn, l.relu, v, l.gb);
-  k_im2colT<<<nblk(v.Vp / 8 * (l.kp / 8)), kT, 0, st>>>(n->act[io], l.cg, v, l.kp, n->colT);
+  k_relu_back<<<dim3((unsigned)std::min<long long>((v.Vp + kT - 1) / kT, 296), (unsigned)(l.cn / 8)), kT, 0, st>>>(
+      gout, out, l.cn, l.relu, v, n->dZ, l.gb);
   UK(cudaGetLastError());
-  UK(cudaMemsetAsync(l.gWT, 0, (size_t)l.kp * l.cn * sizeof(float), st));
-  const int tiles = (l.kp / kBM) * std::max(1, l.cn / 128);
-  const int splitk = std::max(1, std::min((int)(v.Vp / kBK), 296 / tiles));
-  UR(gemm_bf16(n->colT, (int)v.Vp, n->dZT, (int)v.Vp, l.gWT, l.cn, nullptr, l.kp, l.cn, (int)v.Vp, OUT_F32_ATOMIC,
-               splitk, st, n->err));
+  UR(conv_dw(n, li, st));
   if (li == 0) return APHID_UNET_OK;  // no gradient for the input features
   return conv_dx(n, li, n->grad[io], st);
 }
 
 int forward(aphid_unet *n, const float *x, cudaStream_t st) {
   const Vol *V = n->vol;
-  k_pack_in<<<nblk(V[0].Vp * 8), kT, 0, st>>>(x, n->X, n->Y, n->Z, V[0], n->act[A_IN]);
+  k_pack_in<<<nblk(V[0].Vp), kT, 0, st>>>(x, n->X, n->Y, n->Z, V[0], n->act[A_IN]);
   UK(cudaGetLastError());
   auto pool = [&](int a, int b, int lev) {
-    k_pool<<<nblk(V[lev + 1].Vp * (n->ach[a] / 8)), kT, 0, st>>>(n->act[a], n->ach[a], V[lev], V[lev + 1], n->act[b]);
+    k_pool<<<dim3((unsigned)nblk(V[lev + 1].V), (unsigned)(n->ach[a] / 8)), kT, 0, st>>>(n->act[a], V[lev], V[lev + 1], n->act[b]);
   };
-  auto upcat = [&](int low, int skip, int cat, int lev) {
-    k_upcat<<<nblk(V[lev].Vp * (n->ach[cat] / 8)), kT, 0, st>>>(n->act[low], n->ach[low], n->act[skip], n->ach[skip], V[lev],
-                                                          V[lev + 1], n->act[cat]);
+  auto up = [&](int low, int cat, int lev) {
+    k_up<<<dim3((unsigned)nblk(V[lev].V), (unsigned)(n->ach[low] / 8)), kT, 0, st>>>(n->act[low], V[lev], V[lev + 1], n->act[cat]);
   };
   UR(conv_fwd(n, 0, st));
   UR(conv_fwd(n, 1, st));
@@ -634,13 +612,13 @@ int forward(aphid_unet *n, const float *x, cudaStream_t st) {
   pool(S3, P3, 2);
   UR(conv_fwd(n, 6, st));
   UR(conv_fwd(n, 7, st));
-  upcat(A7, S3, CAT3, 2);
+  up(A7, CAT3, 2);
   UR(conv_fwd(n, 8, st));
   UR(conv_fwd(n, 9, st));
-  upcat(A9, S2, CAT2, 1);
+  up(A9, CAT2, 1);
   UR(conv_fwd(n, 10, st));
   UR(conv_fwd(n, 11, st));
-  upcat(A11, S1, CAT1, 0);
+  up(A11, CAT1, 0);
   UR(conv_fwd(n, 12, st));
   UR(conv_fwd(n, 13, st));
   UR(conv_fwd(n, 14, st));
@@ -650,9 +628,7 @@ int forward(aphid_unet *n, const float *x, cudaStream_t st) {
 
 int backward(aphid_unet *n, cudaStream_t st) {
   const Vol *V = n->vol;
-  for (int a = 0; a < A_COUNT; a++)
-    if (n->grad[a]) UK(cudaMemsetAsync(n->grad[a], 0, (size_t)V[n->alev[a]].Vp * n->ach[a] * sizeof(float), st));
-  for (auto &l : n->L) UK(cudaMemsetAsync(l.gb, 0, l.cn * sizeof(float), st));
+  UK(cudaMemsetAsync(n->grad_all, 0, n->grad_bytes, st));
   auto back = [&](int li) {
     const int o = kLayerIO[li][1];
     return o < 0 ? conv_back(n, li, n->gy, nullptr, st) : conv_back(n, li, n->grad[o], n->act[o], st);
@@ -730,21 +706,17 @@ int aphid_unet_create(aphid_unet **out, int X, int Y, int Z, int train, unsigned
   const int ach[A_COUNT] = {8, 16, 16, 16, 32, 32, 32, 64, 64, 64, 128, 128, 192, 64, 64, 96, 32, 32, 48, 16, 16};
   const int alev[A_COUNT] = {0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 3, 2, 2, 2, 1, 1, 1, 0, 0, 0};
   int rc = APHID_UNET_OK;
-  size_t colmax = 0;
   std::mt19937_64 rng(seed);
   for (int li = 0; li < 15 && !rc; li++) {
     Layer l;
     l.cin = kLayerDef[li][0], l.cout = kLayerDef[li][1], l.level = kLayerDef[li][2], l.relu = kLayerDef[li][3];
     l.cg = (int)rup(l.cin, 8), l.cn = (int)rup(l.cout, 16);
     l.nc = l.cg % 32 == 0 ? 32 : l.cg % 48 == 0 ? 48 : 16;
-    l.kp = (int)rup(27LL * l.cg, kBM);
     const size_t nw = 27ULL * l.cin * l.cout;
-    colmax = std::max(colmax, (size_t)n->vol[l.level].Vp * l.kp);
     if ((rc = dalloc(n, &l.W, nw)) || (rc = dalloc(n, &l.b, l.cn)) || (rc = dalloc(n, &l.Wf, 28ULL * l.cg * l.cn)))
       break;
     if (train && ((rc = dalloc(n, &l.mW, nw)) || (rc = dalloc(n, &l.vW, nw)) || (rc = dalloc(n, &l.mb, l.cout)) ||
-                  (rc = dalloc(n, &l.vb, l.cout)) || (rc = dalloc(n, &l.gWT, (size_t)l.kp * l.cn)) ||
-                  (rc = dalloc(n, &l.gb, l.cn)) || (rc = dalloc(n, &l.Wd, 27ULL * rup(l.cg, 16) * l.cn))))
+                  (rc = dalloc(n, &l.vb, l.cout)) || (rc = dalloc(n, &l.Wd, 27ULL * rup(l.cg, 16) * l.cn))))
       break;
     // He-normal initial weights, zero biases
     std::normal_distribution<float> nd(0.f, std::sqrt(2.f / (27.f * l.cin)));
@@ -756,11 +728,23 @@ int aphid_unet_create(aphid_unet **out, int X, int Y, int Z, int train, unsigned
     }
     n->L.push_back(l);
   }
+  size_t gn = 0;  // gradients: activations, then weights and biases
   for (int a = 0; a < A_COUNT && !rc; a++) {
     n->ach[a] = ach[a], n->alev[a] = alev[a];
     const size_t cnt = (size_t)n->vol[alev[a]].Vp * ach[a];
-    rc = dalloc(n, &n->act[a], cnt);
-    if (!rc && train && a != A_IN) rc = dalloc(n, &n->grad[a], cnt);
+    if (a != S1 && a != S2 && a != S3) rc = dalloc(n, &n->act[a], cnt);
+    if (a != A_IN) gn += cnt;
+  }
+  // a skip is the lower planes of its concatenation
+  for (auto &sc : {std::pair<int, int>{S1, CAT1}, {S2, CAT2}, {S3, CAT3}})
+    if (!rc) n->act[sc.first] = n->act[sc.second] + (size_t)n->vol[alev[sc.second]].Vp * (ach[sc.second] - ach[sc.first]);
+  for (auto &l : n->L) gn += 27ULL * l.cg * l.cn + l.cn, n->nparam += l.nparam();
+  if (!rc && train && !(rc = dalloc(n, &n->grad_all, gn)) && !(rc = dalloc(n, &n->gout, n->nparam))) {
+    n->grad_bytes = gn * sizeof(float);
+    float *g = n->grad_all;
+    for (int a = 0; a < A_COUNT; a++)
+      if (a != A_IN) n->grad[a] = g, g += (size_t)n->vol[alev[a]].Vp * ach[a];
+    for (auto &l : n->L) l.gWT = g, g += 27ULL * l.cg * l.cn, l.gb = g, g += l.cn;
   }
   if (!rc) rc = dalloc(n, &n->y, (size_t)n->vol[0].Vp * 16);
   if (!rc) rc = dalloc(n, &n->err, 1);
@@ -771,9 +755,7 @@ int aphid_unet_create(aphid_unet **out, int X, int Y, int Z, int train, unsigned
       dzmax = std::max(dzmax, (size_t)n->vol[l.level].Vp * l.cn);
     }
     if (!rc) rc = dalloc(n, &n->gy, (size_t)n->vol[0].Vp * 16);
-    if (!rc) rc = dalloc(n, &n->colT, colmax);
     if (!rc) rc = dalloc(n, &n->dZ, dzmax);
-    if (!rc) rc = dalloc(n, &n->dZT, dzmax);
   }
   if (!rc) rc = cast_weights(n, 0);
   if (!rc && cudaDeviceSynchronize() != cudaSuccess) rc = set_err(APHID_UNET_ERR_CUDA, "unet_create: initialisation");
@@ -829,7 +811,7 @@ int aphid_unet_forward(aphid_unet *n, const float *x, float *y, void *stream) {
   if (!n || !x || !y) return set_err(APHID_UNET_ERR_BADARG, "unet_forward: null");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   UR(forward(n, x, st));
-  k_unpack_out<<<nblk((long long)n->X * n->Y * n->Z * 8), kT, 0, st>>>(n->y, n->X, n->Y, n->Z, n->vol[0], y);
+  k_unpack_out<<<nblk((long long)n->X * n->Y * n->Z * 2), kT, 0, st>>>(n->y, n->X, n->Y, n->Z, n->vol[0], y);
   UK(cudaGetLastError());
   return check_err(n, st);
 }
@@ -866,19 +848,12 @@ int aphid_unet_train_step(aphid_unet *n, const float *x, const float *target, co
 int aphid_unet_get_grads(aphid_unet *n, float *host) {
   if (!n || !host || !n->train) return set_err(APHID_UNET_ERR_BADARG, "unet_get_grads: no training buffers");
   size_t o = 0;
-  float *tmp = nullptr;
-  size_t maxn = 0;
-  for (auto &l : n->L) maxn = std::max(maxn, (size_t)l.nparam());
-  UK(cudaMalloc(&tmp, maxn * sizeof(float)));
   for (auto &l : n->L) {
-    k_grad_out<<<nblk(l.nparam()), kT>>>(l.gWT, l.gb, l.cin, l.cg, l.cout, l.cn, tmp);
-    if (cudaMemcpy(host + o, tmp, l.nparam() * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) {
-      cudaFree(tmp);
-      return set_err(APHID_UNET_ERR_CUDA, "unet_get_grads: copy");
-    }
+    k_grad_out<<<nblk(l.nparam()), kT>>>(l.gWT, l.gb, l.cin, l.cg, l.cout, l.cn, n->gout + o);
     o += l.nparam();
   }
-  cudaFree(tmp);
+  UK(cudaGetLastError());
+  UK(cudaMemcpy(host, n->gout, o * sizeof(float), cudaMemcpyDeviceToHost));
   return APHID_UNET_OK;
 }
 

@@ -1,6 +1,6 @@
 // unet_conv.cuh -- the 3 x 3 x 3 convolutions of the initial-guess network as
-// implicit GEMMs on the sm_100a tensor cores (tcgen05): forward, and the data
-// gradient.  No column matrix: a block brings the voxels of its tile with a
+// implicit GEMMs on the sm_100a tensor cores (tcgen05): forward, data gradient
+// and weight gradient.  No column matrix: a block brings the voxels of its tile with a
 // one-voxel halo into shared memory once, and every tap's operand is the same
 // memory read from a shifted start address.
 //
@@ -402,6 +402,110 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_dx(const __grid_constant_
         o.z += sum[p * NC + 4 * q + 2];
         o.w += sum[p * NC + 4 * q + 3];
         g[q] = o;
+      }
+    }
+  }
+  if (!ok && err) atomicExch(err, 1);
+  conv_exit(tmem, kCols);
+}
+
+// Weight gradient: gW[tap * C + c][n] += sum over the voxels of in[r + d_tap][c]
+// dz[r][n], CH planes of 8 input channels, CN outputs.  The voxels are the K
+// dimension, so both operands are MN-major: 8 voxels x 8 channels of a plane are
+// 128 contiguous bytes, one core matrix.  The 128 rows of a block are 16 slots of 8
+// channels, a slot being a (dy, dz) shift of a plane, staged as 16 rows of 10
+// voxels; the three dx are three products from start addresses 16 bytes apart into
+// three accumulators, so a staged slot serves three taps (single taps staged at 8
+// voxels a row copy 2.4 x the bytes).  Blocks along y split the tiles of the
+// volume and add their sums with vector reductions, as a split-K GEMM would.
+// It is bound by the copies of the shifted slots from L2 (9 x the activations).
+// Against 64-bit sums of the same operands (16 -> 16 channels of 72 x 72 x 56) it
+// is off by 4.0e-6 where all terms are positive and by 1.4e-6 where their signs
+// are mixed; the GEMM over a transposed column matrix by 1.1e-5 and 2.8e-6 (tensor
+// memory truncates: the error grows with the terms of one accumulator).  The 15
+// weight gradients of a training step take 0.25 ms; 1.2 with the column matrices.
+template <int CH, int CN>
+struct DwShape {
+  static constexpr int kSlots = 9 * CH, kGroups = (kSlots + 15) / 16;
+  static constexpr uint32_t slot_b = kTY * kRowB, plane_b = kTX * kTY * 16;
+  static constexpr uint32_t stage_b = 16 * slot_b + CN / 8 * plane_b;
+  static constexpr int ST = CN <= 32 ? 2 : 3;  // two blocks per SM, or one with a deeper ring
+  static constexpr size_t shm = 128 + ST * stage_b + 256;
+};
+template <int CH, int CN>
+__global__ void __launch_bounds__(kConvThreads) k_conv_dw(const __grid_constant__ CUtensorMap map_in,
+                                                          const __grid_constant__ CUtensorMap map_dz, const ConvArgs a,
+                                                          int tiles, float *__restrict__ gw, int *err) {
+  using D = DwShape<CH, CN>;
+  extern __shared__ unsigned char cs_raw[];
+  constexpr uint32_t kCols = tmem_cols(3 * CN);
+  uint32_t tmem;
+  const ConvShm s = conv_init<0, 0, D::ST * D::stage_b, kCols>(cs_raw, tmem);
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int slot0 = blockIdx.x * 16, used = min(16, D::kSlots - slot0);
+  bool ok = true;
+  if (warp == 4) {
+    // lane q < used copies slot q, the next CN / 8 lanes the planes of dz
+    const int c = lane < used ? (slot0 + lane) % CH : lane - used, sh = (slot0 + lane) / CH;
+    const int sy = lane < used ? sh % 3 - 1 : 0, sz = lane < used ? sh / 3 - 1 : 0, sx = lane < used ? 1 : 0;
+    int st = 0, lap = 0;
+    for (int i = blockIdx.y; i < tiles; i += gridDim.y) {
+      if (lap > 0 && ok) ok = g_mbar_wait(gsm(&s.empty[st]), (uint32_t)((lap - 1) & 1));
+      const int x = i % a.tx * kTX, y = i / a.tx % a.ty * kTY, z = i / (a.tx * a.ty);
+      const uint32_t base = gsm(s.w) + st * D::stage_b, bar = gsm(&s.full[st]);
+      if (lane == 0) g_mbar_expect(bar, used * D::slot_b + CN / 8 * D::plane_b);
+      __syncwarp();
+      if (lane < used)
+        g_tma_load4(base + lane * D::slot_b, &map_in, (x - sx) * 8, y + sy, z + sz, c, bar);
+      else if (lane < used + CN / 8)
+        g_tma_load4(base + 16 * D::slot_b + c * D::plane_b, &map_dz, x * 8, y, z, c, bar);
+      if (++st == D::ST) st = 0, lap++;
+    }
+  } else if (warp == 5) {
+    // both operands MN-major (bits 15, 16)
+    constexpr uint32_t idesc = idesc_bf16(kBM, CN) | (1u << 15) | (1u << 16);
+    const bool lead = elect_one();
+    int st = 0, lap = 0;
+    uint32_t acc = 0;
+    for (int i = blockIdx.y; i < tiles; i += gridDim.y) {
+      if (ok) ok = g_mbar_wait(gsm(&s.full[st]), (uint32_t)(lap & 1));
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t base = gsm(s.w) + st * D::stage_b;
+      const uint64_t da = smem_desc(base, kRowB, D::slot_b), db = smem_desc(base + 16 * D::slot_b, kTX * 16, D::plane_b);
+      if (lead) {
+#pragma unroll
+        for (int k = 0; k < kTY / 2; k++) {  // 16 voxels: two rows of 8
+#pragma unroll
+          for (int dx = 0; dx < 3; dx++)
+            mma_f16(tmem + dx * CN, da + ((k * 2 * kRowB + dx * 16) >> 4), db + (k * 2 * kTX * 16 >> 4), idesc, acc | (k > 0));
+        }
+        mma_commit(gsm(&s.empty[st]));
+      }
+      acc = 1;
+      if (++st == D::ST) st = 0, lap++;
+    }
+    if (lead) mma_commit(gsm(s.tfull));
+  }
+  __syncwarp();
+  if (warp < 4) {
+    ok = g_mbar_wait(gsm(s.tfull), 0u) && ok;
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const int row = warp * 32 + lane, slot = slot0 + row / 8;
+    const uint32_t at = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+    for (int dx = 0; dx < 3; dx++) {
+      float *o = gw + ((long long)((slot / CH) * 3 + dx) * (CH * 8) + slot % CH * 8 + row % 8) * CN;
+#pragma unroll 1
+      for (int c0 = 0; c0 < CN; c0 += 8) {
+        float f[8];
+        __syncwarp();
+        tmem_ld8(at + dx * CN + c0, f);
+        tmem_ld_wait();
+        if (slot < D::kSlots && ok) {
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(o + c0), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(o + c0 + 4), "f"(f[4]), "f"(f[5]), "f"(f[6]), "f"(f[7]) : "memory");
+        }
       }
     }
   }
