@@ -12,7 +12,7 @@
 // also read; at 166 registers and 4 warps per block that kernel is
 // latency-bound (1.1 TB/s).  Here a 32 x 8 node tile marches along k:
 //   - per z-plane, the block stages x, the k^2 of the Ax, Ay and Phi blocks
-//     (7 arrays of 34 x 10 values: the tile with a one-node halo, global
+//     (7 arrays of up to 34 x 10 values: the tile with a one-node halo, global
 //     indices clamped to each block's range, which is exactly the clamping
 //     of the reference's neighbour indices), so every x/y neighbour is a
 //     shared-memory read;
@@ -22,7 +22,15 @@
 // Planes are staged by cp.async (global -> shared, no register staging) two
 // planes ahead of their use, in a ring of three buffers (planes k, k+1 and
 // k+2 in flight), so the loads of the next planes overlap the rows of this
-// one.  One block of 256 threads, 112 KB of shared memory, two blocks per SM.
+// one.  Two blocks of 256 threads per SM, 115 KB of shared memory each.
+// Bound by latency (16 warps per SM, about 600 instructions per node of which a
+// third FP64): what would sit on a plane's critical path is brought in before
+// it -- the addresses of the staged values and the planes' factors with their
+// divisions from shared-memory tables, k^2 of Az a plane ahead -- and nothing is
+// spilled: the staging leaves 28 KB of L1, so spilled registers went to L2.
+// 161 x 161 x 129 nodes: 235 -> 187 us (48 B per unknown at the copy rate: 98);
+// 65 x 65 x 49: 19.7 -> 15.2.  One thread per node for A's rows and one for Phi's
+// (32 warps, 64 registers) spilled and took 415; one block per SM 218.
 // Global traffic per node and plane: x and k^2 read once (plus the halo,
 // 33%), y written once: the 48 B per unknown of the operator.
 #pragma once
@@ -32,10 +40,18 @@ namespace aphid {
 
 constexpr int kAI = 32, kAJ = 8, kAThreads = kAI * kAJ;
 constexpr int kAW = kAI + 2, kAH = kAJ + 2, kAN = kAW * kAH;  // staged plane with halo: 34 x 10
-constexpr int kAArrays = 7;                                   // x: Ax Ay Az Phi; k^2: Ax Ay Phi
-constexpr int kABufs = 3;
-constexpr size_t kApplyShm = kABufs * (size_t)kAArrays * kAN * sizeof(double2);
-enum { SA_AX = 0, SA_AY, SA_AZ, SA_PH, SK_AX, SK_AY, SK_PH };
+constexpr int kABufs = 3, kAMaxKz = 32;                       // staging buffers, deepest slab of apply_tiles
+// x: Ax Ay Az Phi with the halo; k^2 of Phi without the row below, of Ay without
+// the row above, of Ax without both (never read): two blocks per SM need every
+// one of these rows
+enum { SA_AX = 0, SA_AY = kAN, SA_AZ = 2 * kAN, SA_PH = 3 * kAN, SK_PH = 4 * kAN - kAW, SK_AY = SK_PH + kAN,
+       SK_AX = SK_AY + kAN - 2 * kAW };
+constexpr int kAPlane = SK_AX + kAN - kAW;
+// what a block keeps beside the staged planes: the factors of the slab's planes,
+// and where the staged values of plane 0 lie in [Ax|Ay|Az|Phi]
+struct ApplyZ { double n4, n5, dc, d, e2, e3, rdc, rd; };
+constexpr size_t kApplyShm = kABufs * (size_t)kAPlane * sizeof(double2) + kAMaxKz * sizeof(ApplyZ) + kAN * sizeof(uint4);
+static_assert(2 * (kApplyShm + 256 + 1024) <= 233472, "two blocks per SM");
 
 // Plane tiles of k_apply64s: kAI x kAJ nodes, kz planes per block.
 inline Tiles apply_tiles(int nx, int ny, int nz, int sms) {
@@ -77,7 +93,9 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
                                                                   double2 *__restrict__ out, Scal64 *sc,
                                                                   double2 *eps_out, double *part, unsigned *cnt) {
   if (MODE == kApplyQmr && sc->done) return;
-  extern __shared__ __align__(16) double2 sa[];  // [kABufs][kAArrays][kAN]
+  extern __shared__ __align__(16) double2 sa[];  // [kABufs][kAPlane], zr, at
+  ApplyZ *zr = reinterpret_cast<ApplyZ *>(sa + kABufs * kAPlane);
+  uint4 *at = reinterpret_cast<uint4 *>(zr + kAMaxKz);
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   int b = blockIdx.x;
   const int bi = b % tl.ti;
@@ -90,42 +108,66 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
   const bool live = i < nx && j < ny;
   const int me = (ty + 1) * kAW + (tx + 1);  // own node in a staged plane
 
-  // global index of staged array a at (gi, gj) of plane m, clamped to the
-  // block's own range (the reference's min/max neighbour indices)
-  auto src = [&](int a, int gi, int gj, int m) -> const double2 * {
-    const int c = a < 4 ? a : (a == SK_PH ? 3 : a - 4);
-    const int il = c == 0 ? nx - 2 : nx - 1, jl = c == 1 ? ny - 2 : ny - 1;
-    gi = min(max(gi, 0), il);
-    gj = min(max(gj, 0), jl);
-    if (c == 2) m = min(m, nz - 2);
-    const long long t = c == 0 ? ixx(g, gi, gj, m) : (c == 1 ? ixy(g, gi, gj, m) : (c == 2 ? ixz(g, gi, gj, m) : ixp(g, gi, gj, m)));
-    return (a < 4 ? in : k2) + t;
-  };
+  // where the four blocks' values at the staged positions lie in plane 0, indices
+  // clamped to each block's own range (the reference's min/max neighbour
+  // indices); 32 bits hold them: 2^32 unknowns would take 206 GB for x, k^2 and y.
+  // In shared memory, like the factors of the planes below: every spilled
+  // register goes to L2, the staging leaves 28 KB of the SM's memory as L1
+  for (int p = threadIdx.x; p < kAN; p += kAThreads) {
+    const int gi = max(i0 - 1 + p % kAW, 0), gj = max(j0 - 1 + p / kAW, 0);
+    const int ci = min(gi, nx - 1), cj = min(gj, ny - 1);
+    at[p] = make_uint4((unsigned)ixx(g, min(gi, nx - 2), cj, 0), (unsigned)ixy(g, ci, min(gj, ny - 2), 0),
+                       (unsigned)ixz(g, ci, cj, 0), (unsigned)ixp(g, ci, cj, 0));
+  }
+  if (threadIdx.x < k1 - k0) {
+    // x / d becomes x (1/d): within an ulp, and no FP64 divide in the plane loop
+    const int k = k0 + threadIdx.x;
+    ApplyZ z;
+    z.n4 = g.ax[2].n4[k], z.n5 = g.ax[2].n5[k], z.dc = g.ax[2].dc[k], z.d = g.ax[2].d[k + 1];
+    z.e2 = k < nz - 1 ? g.ax[2].e2[k] : 0.0, z.e3 = k < nz - 1 ? g.ax[2].e3[k] : 0.0;
+    z.rdc = 1.0 / z.dc, z.rd = 1.0 / z.d;
+    zr[threadIdx.x] = z;
+  }
+  const unsigned pn = (unsigned)nx * ny, px = (unsigned)(nx - 1) * ny, py = (unsigned)nx * (ny - 1);
+  __syncthreads();
+  const uint4 *const own = at + me;
   // start staging plane m into buffer s (cp.async, one commit group per
   // plane, possibly empty): all arrays with halo, or (own_only) the values at
   // the block's own nodes that the plane below needs; nothing when m is past
   // the slab's last plane + 1 or the mesh
   auto stage = [&](int s, int m) {
-    double2 *B = sa + (size_t)s * kAArrays * kAN;
+    double2 *B = sa + s * kAPlane;
     if (m < nz && m < k1) {
+      const unsigned mx = px * m, my = py * m, mz = pn * min(m, nz - 2), mp = pn * m;
 #pragma unroll
       for (int q = 0; q < (kAN + kAThreads - 1) / kAThreads; q++) {
         const int p = threadIdx.x + q * kAThreads;
         if (p < kAN) {
-          const int gi = i0 - 1 + p % kAW, gj = j0 - 1 + p / kAW;
-#pragma unroll
-          for (int a = 0; a < kAArrays; a++) cp_async16(B + a * kAN + p, src(a, gi, gj, m));
+          const uint4 t = at[p];
+          cp_async16(B + SA_AX + p, in + (t.x + mx));
+          cp_async16(B + SA_AY + p, in + (t.y + my));
+          cp_async16(B + SA_AZ + p, in + (t.z + mz));
+          cp_async16(B + SA_PH + p, in + (t.w + mp));
+          if (p >= kAW) cp_async16(B + SK_PH + p, k2 + (t.w + mp));
+          if (p < kAN - kAW) cp_async16(B + SK_AY + p, k2 + (t.y + my));
+          if (p >= kAW && p < kAN - kAW) cp_async16(B + SK_AX + p, k2 + (t.x + mx));
         }
       }
     } else if (m < nz && m == k1) {
-      const int as[5] = {SA_AX, SA_AY, SA_AZ, SA_PH, SK_PH};
-#pragma unroll
-      for (int q = 0; q < 5; q++) cp_async16(B + as[q] * kAN + me, src(as[q], i, j, m));
+      const uint4 t = *own;
+      cp_async16(B + SA_AX + me, in + (t.x + px * m));
+      cp_async16(B + SA_AY + me, in + (t.y + py * m));
+      cp_async16(B + SA_AZ + me, in + (t.z + pn * min(m, nz - 2)));
+      cp_async16(B + SA_PH + me, in + (t.w + pn * m));
+      cp_async16(B + SK_PH + me, k2 + (t.w + pn * m));
     }
     cp_async_commit();
   };
 
-  const Axis &X = g.ax[0], &Y = g.ax[1], &Z = g.ax[2];
+  stage(0, k0);
+  stage(1, k0 + 1);
+
+  const Axis &X = g.ax[0], &Y = g.ax[1];
   const int ic = min(i, nx - 1), jc = min(j, ny - 1);
   const double xn4 = X.n4[ic], xn5 = X.n5[ic], yn4 = Y.n4[jc], yn5 = Y.n5[jc];
   const double dxc = X.dc[ic], dyc = Y.dc[jc];
@@ -135,45 +177,44 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
   const bool hx = live && i < nx - 1, hy = live && j < ny - 1;
   const bool pxy = live && i > 0 && i < nx - 1 && j > 0 && j < ny - 1;
 
-  // plane k0-1 (clamped at 0) at the own node: x of the four blocks and k^2 of Az
-  double2 axm, aym, azm, phm, kazm;
+  // plane k0-1 (clamped at 0) at the own node: x of the four blocks and k^2 of Az;
+  // k^2 of Az one plane ahead
+  double2 axm, aym, azm, phm, kazm, kaz;
   {
-    const int m = max(k0 - 1, 0);
-    axm = __ldg(src(SA_AX, i, j, m));
-    aym = __ldg(src(SA_AY, i, j, m));
-    azm = __ldg(src(SA_AZ, i, j, m));
-    phm = __ldg(src(SA_PH, i, j, m));
-    kazm = __ldg(k2 + ixz(g, min(i, nx - 1), min(j, ny - 1), min(m, nz - 2)));
+    const unsigned m = max(k0 - 1, 0);
+    const uint4 t = *own;
+    axm = __ldg(in + (t.x + px * m));
+    aym = __ldg(in + (t.y + py * m));
+    azm = __ldg(in + (t.z + pn * m));
+    phm = __ldg(in + (t.w + pn * m));
+    kazm = __ldg(k2 + (t.z + pn * m));
+    kaz = __ldg(k2 + (t.z + pn * min(k0, nz - 2)));
   }
-  stage(0, k0);
-  stage(1, k0 + 1);
-
   double ea = 0.0, eb = 0.0;
   for (int k = k0; k < k1; k++) {
     const int s = (k - k0) % kABufs, sn = (k - k0 + 1) % kABufs;
     const bool has_next = k + 1 < nz;
     stage((k - k0 + 2) % kABufs, k + 2);  // into the buffer plane k-1 used
-    const double2 kaz = __ldg(k2 + ixz(g, min(i, nx - 1), min(j, ny - 1), min(k, nz - 2)));
+    const double2 kaz_n = __ldg(k2 + (own->z + pn * min(k + 1, nz - 2)));
     cp_async_wait<1>();  // this thread's copies of planes k and k+1 have landed
     __syncthreads();     // ... and everyone's
-    const double2 *C = sa + (size_t)s * kAArrays * kAN;
-    const double2 *Nx = has_next ? sa + (size_t)sn * kAArrays * kAN : C;  // plane k+1, clamped at nz-1
+    const double2 *C = sa + s * kAPlane + me;
+    const double2 *Nx = has_next ? sa + sn * kAPlane + me : C;  // plane k+1, clamped at nz-1
     // shared-memory values are read where they are used (short live ranges)
-    auto cur = [&](int a, int off) { return C[a * kAN + me + off]; };
-    auto nxt = [&](int a) { return Nx[a * kAN + me]; };
+    auto cur = [&](int a, int off) { return C[a + off]; };
+    auto nxt = [&](int a) { return Nx[a]; };
     const double2 phc = cur(SA_PH, 0), kpc = cur(SK_PH, 0);
-    const double zn4 = Z.n4[k], zn5 = Z.n5[k], dzc = Z.dc[k], rdzc = 1.0 / dzc, rdzk = 1.0 / Z.d[k + 1];
+    const ApplyZ &z = zr[k - k0];
     double2 e = make_double2(0.0, 0.0);
     if (live) {
-      const long long pc = ixp(g, i, j, k);
-      double2 op = make_double2(0.0, 0.0);
+            double2 op = make_double2(0.0, 0.0);
       if (pxy && k > 0 && k < nz - 1) {
-        const double vol = dxc * dyc * dzc;
+        const double vol = dxc * dyc * z.dc;
         const double2 s1 = kpc;
         const double2 s2 = cur(SK_AX, 0), s3 = cur(SK_AX, -1), s4 = cur(SK_AY, 0);
         const double2 s5 = cur(SK_AY, -kAW), s6 = kaz, s7 = kazm;
         const double2 c2 = rmul(xn4, s2), c3 = rmul(xn5, s3), c4 = rmul(yn4, s4);
-        const double2 c5 = rmul(yn5, s5), c6 = rmul(zn4, s6), c7 = rmul(zn5, s7);
+        const double2 c5 = rmul(yn5, s5), c6 = rmul(z.n4, s6), c7 = rmul(z.n5, s7);
         double2 sum = cadd(cadd(cadd(cadd(cadd(c2, c3), c4), c5), c6), c7);
         const double2 c1 = cadd(cneg(sum), cmul(s1, s1));
         double2 t = cmul(c1, phc);
@@ -186,7 +227,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         const double2 acc = rmul(vol, t);
         const double2 d2 = rmul(rdxc, csub(s2, s1)), d3 = cneg(rmul(rdxc, csub(s3, s1)));
         const double2 d4 = rmul(rdyc, csub(s4, s1)), d5 = cneg(rmul(rdyc, csub(s5, s1)));
-        const double2 d6 = rmul(rdzc, csub(s6, s1)), d7 = cneg(rmul(rdzc, csub(s7, s1)));
+        const double2 d6 = rmul(z.rdc, csub(s6, s1)), d7 = cneg(rmul(z.rdc, csub(s7, s1)));
         double2 u = cmul(d2, cur(SA_AX, 0));
         u = cadd(u, cmul(d3, cur(SA_AX, -1)));
         u = cadd(u, cmul(d4, cur(SA_AY, 0)));
@@ -195,46 +236,46 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         u = cadd(u, cmul(d7, azm));
         op = cadd(acc, rmul(vol, u));
       }
-      out[pc] = op;
+      out[own->w + pn * k] = op;
       e = cmul(phc, op);
       if (hx) {
         const double c2 = X.e2[i], c3 = X.e3[i], dxi = X.d[i + 1];
-        const double vol = dxi * dyc * dzc;
+        const double vol = dxi * dyc * z.dc;
         const double2 kx = cur(SK_AX, 0), kp2 = cur(SK_PH, 1), axc = cur(SA_AX, 0);
-        const double sum = c2 + c3 + yn4 + yn5 + zn4 + zn5;
+        const double sum = c2 + c3 + yn4 + yn5 + z.n4 + z.n5;
         const double2 c1 = make_double2(-sum + kx.x, kx.y);
         double2 t = cmul(c1, axc);
         t = cadd(t, rmul(c2, cur(SA_AX, 1)));
         t = cadd(t, rmul(c3, cur(SA_AX, -1)));
         t = cadd(t, rmul(yn4, cur(SA_AX, kAW)));
         t = cadd(t, rmul(yn5, cur(SA_AX, -kAW)));
-        t = cadd(t, rmul(zn4, nxt(SA_AX)));
-        t = cadd(t, rmul(zn5, axm));
+        t = cadd(t, rmul(z.n4, nxt(SA_AX)));
+        t = cadd(t, rmul(z.n5, axm));
         const double2 gr = rmul(rdxi, csub(cmul(cur(SA_PH, 1), csub(kp2, kx)), cmul(phc, csub(kpc, kx))));
         const double2 ox = rmul(vol, cadd(t, gr));
-        out[ixx(g, i, j, k)] = ox;
+        out[own->x + px * k] = ox;
         e = cadd(e, cmul(axc, ox));
       }
       if (hy) {
         const double c2 = Y.e2[j], c3 = Y.e3[j], dyj = Y.d[j + 1];
-        const double vol = dxc * dyj * dzc;
+        const double vol = dxc * dyj * z.dc;
         const double2 ky = cur(SK_AY, 0), kp2 = cur(SK_PH, kAW), ayc = cur(SA_AY, 0);
-        const double sum = c2 + c3 + xn4 + xn5 + zn4 + zn5;
+        const double sum = c2 + c3 + xn4 + xn5 + z.n4 + z.n5;
         const double2 c1 = make_double2(-sum + ky.x, ky.y);
         double2 t = cmul(c1, ayc);
         t = cadd(t, rmul(c2, cur(SA_AY, kAW)));
         t = cadd(t, rmul(c3, cur(SA_AY, -kAW)));
         t = cadd(t, rmul(xn4, cur(SA_AY, 1)));
         t = cadd(t, rmul(xn5, cur(SA_AY, -1)));
-        t = cadd(t, rmul(zn4, nxt(SA_AY)));
-        t = cadd(t, rmul(zn5, aym));
+        t = cadd(t, rmul(z.n4, nxt(SA_AY)));
+        t = cadd(t, rmul(z.n5, aym));
         const double2 gr = rmul(rdyj, csub(cmul(cur(SA_PH, kAW), csub(kp2, ky)), cmul(phc, csub(kpc, ky))));
         const double2 oy = rmul(vol, cadd(t, gr));
-        out[ixy(g, i, j, k)] = oy;
+        out[own->y + py * k] = oy;
         e = cadd(e, cmul(ayc, oy));
       }
       if (k < nz - 1) {
-        const double c2 = Z.e2[k], c3 = Z.e3[k], dzk = Z.d[k + 1];
+        const double c2 = z.e2, c3 = z.e3, dzk = z.d;
         const double vol = dxc * dyc * dzk;
         const double2 kz = kaz, kp2 = nxt(SK_PH), azc = cur(SA_AZ, 0);
         const double sum = c2 + c3 + xn4 + xn5 + yn4 + yn5;
@@ -246,9 +287,9 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         t = cadd(t, rmul(xn5, cur(SA_AZ, -1)));
         t = cadd(t, rmul(yn4, cur(SA_AZ, kAW)));
         t = cadd(t, rmul(yn5, cur(SA_AZ, -kAW)));
-        const double2 gr = rmul(rdzk, csub(cmul(nxt(SA_PH), csub(kp2, kz)), cmul(phc, csub(kpc, kz))));
+        const double2 gr = rmul(z.rd, csub(cmul(nxt(SA_PH), csub(kp2, kz)), cmul(phc, csub(kpc, kz))));
         const double2 oz = rmul(vol, cadd(t, gr));
-        out[ixz(g, i, j, k)] = oz;
+        out[own->z + pn * k] = oz;
         e = cadd(e, cmul(azc, oz));
       }
     }
@@ -259,6 +300,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
     azm = cur(SA_AZ, 0);
     phm = phc;
     kazm = kaz;
+    kaz = kaz_n;
     __syncthreads();  // buffer s is free for plane k+3
   }
   cp_async_wait<0>();
