@@ -28,8 +28,8 @@
 // it -- the addresses of the staged values and the planes' factors with their
 // divisions from shared-memory tables, k^2 of Az a plane ahead -- and nothing is
 // spilled: the staging leaves 28 KB of L1, so spilled registers went to L2.
-// 161 x 161 x 129 nodes: 235 -> 187 us (48 B per unknown at the copy rate: 98);
-// 65 x 65 x 49: 19.7 -> 15.2.  One thread per node for A's rows and one for Phi's
+// 161 x 161 x 129 nodes: 235 -> 180 us (48 B per unknown at the copy rate: 98);
+// 65 x 65 x 49: 19.7 -> 14.8.  One thread per node for A's rows and one for Phi's
 // (32 warps, 64 registers) spilled and took 415; one block per SM 218.
 // Global traffic per node and plane: x and k^2 read once (plus the halo,
 // 33%), y written once: the 48 B per unknown of the operator.
@@ -50,7 +50,8 @@ constexpr int kAPlane = SK_AX + kAN - kAW;
 // what a block keeps beside the staged planes: the factors of the slab's planes,
 // and where the staged values of plane 0 lie in [Ax|Ay|Az|Phi]
 struct ApplyZ { double n4, n5, dc, d, e2, e3, rdc, rd; };
-constexpr size_t kApplyShm = kABufs * (size_t)kAPlane * sizeof(double2) + kAMaxKz * sizeof(ApplyZ) + kAN * sizeof(uint4);
+constexpr size_t kApplyShm = kABufs * (size_t)kAPlane * sizeof(double2) + kAMaxKz * sizeof(ApplyZ) + kAN * sizeof(uint2) + kAN * sizeof(unsigned) +
+                             3 * (kAI + kAJ) * sizeof(double);
 static_assert(2 * (kApplyShm + 256 + 1024) <= 233472, "two blocks per SM");
 
 // Plane tiles of k_apply64s: kAI x kAJ nodes, kz planes per block.
@@ -95,7 +96,9 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
   if (MODE == kApplyQmr && sc->done) return;
   extern __shared__ __align__(16) double2 sa[];  // [kABufs][kAPlane], zr, at
   ApplyZ *zr = reinterpret_cast<ApplyZ *>(sa + kABufs * kAPlane);
-  uint4 *at = reinterpret_cast<uint4 *>(zr + kAMaxKz);
+  double *xe = reinterpret_cast<double *>(zr + kAMaxKz), *ye = xe + 3 * kAI;  // e2, e3, d of the tile's columns, rows
+  uint2 *axy = reinterpret_cast<uint2 *>(ye + 3 * kAJ);
+  unsigned *az = reinterpret_cast<unsigned *>(axy + kAN);
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   int b = blockIdx.x;
   const int bi = b % tl.ti;
@@ -116,8 +119,16 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
   for (int p = threadIdx.x; p < kAN; p += kAThreads) {
     const int gi = max(i0 - 1 + p % kAW, 0), gj = max(j0 - 1 + p / kAW, 0);
     const int ci = min(gi, nx - 1), cj = min(gj, ny - 1);
-    at[p] = make_uint4((unsigned)ixx(g, min(gi, nx - 2), cj, 0), (unsigned)ixy(g, ci, min(gj, ny - 2), 0),
-                       (unsigned)ixz(g, ci, cj, 0), (unsigned)ixp(g, ci, cj, 0));
+    axy[p] = make_uint2((unsigned)ixx(g, min(gi, nx - 2), cj, 0), (unsigned)ixy(g, ci, min(gj, ny - 2), 0));
+    az[p] = (unsigned)ixz(g, ci, cj, 0);
+  }
+  const unsigned zp = (unsigned)(g.op - g.oz);  // Phi lies like Az
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + kAI) {
+    const int q = threadIdx.x - 64, n = min(i0 + q, nx - 2);
+    xe[q] = g.ax[0].e2[n], xe[kAI + q] = g.ax[0].e3[n], xe[2 * kAI + q] = g.ax[0].d[n + 1];
+  } else if (threadIdx.x >= 96 && threadIdx.x < 96 + kAJ) {
+    const int q = threadIdx.x - 96, n = min(j0 + q, ny - 2);
+    ye[q] = g.ax[1].e2[n], ye[kAJ + q] = g.ax[1].e3[n], ye[2 * kAJ + q] = g.ax[1].d[n + 1];
   }
   if (threadIdx.x < k1 - k0) {
     // x / d becomes x (1/d): within an ulp, and no FP64 divide in the plane loop
@@ -130,7 +141,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
   }
   const unsigned pn = (unsigned)nx * ny, px = (unsigned)(nx - 1) * ny, py = (unsigned)nx * (ny - 1);
   __syncthreads();
-  const uint4 *const own = at + me;
+  auto at = [&](int p) { return make_uint4(axy[p].x, axy[p].y, az[p], az[p] + zp); };
   // start staging plane m into buffer s (cp.async, one commit group per
   // plane, possibly empty): all arrays with halo, or (own_only) the values at
   // the block's own nodes that the plane below needs; nothing when m is past
@@ -143,7 +154,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
       for (int q = 0; q < (kAN + kAThreads - 1) / kAThreads; q++) {
         const int p = threadIdx.x + q * kAThreads;
         if (p < kAN) {
-          const uint4 t = at[p];
+          const uint4 t = at(p);
           cp_async16(B + SA_AX + p, in + (t.x + mx));
           cp_async16(B + SA_AY + p, in + (t.y + my));
           cp_async16(B + SA_AZ + p, in + (t.z + mz));
@@ -154,7 +165,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         }
       }
     } else if (m < nz && m == k1) {
-      const uint4 t = *own;
+      const uint4 t = at(me);
       cp_async16(B + SA_AX + me, in + (t.x + px * m));
       cp_async16(B + SA_AY + me, in + (t.y + py * m));
       cp_async16(B + SA_AZ + me, in + (t.z + pn * min(m, nz - 2)));
@@ -182,7 +193,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
   double2 axm, aym, azm, phm, kazm, kaz;
   {
     const unsigned m = max(k0 - 1, 0);
-    const uint4 t = *own;
+    const uint4 t = at(me);
     axm = __ldg(in + (t.x + px * m));
     aym = __ldg(in + (t.y + py * m));
     azm = __ldg(in + (t.z + pn * m));
@@ -195,7 +206,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
     const int s = (k - k0) % kABufs, sn = (k - k0 + 1) % kABufs;
     const bool has_next = k + 1 < nz;
     stage((k - k0 + 2) % kABufs, k + 2);  // into the buffer plane k-1 used
-    const double2 kaz_n = __ldg(k2 + (own->z + pn * min(k + 1, nz - 2)));
+    const double2 kaz_n = __ldg(k2 + (az[me] + pn * min(k + 1, nz - 2)));
     cp_async_wait<1>();  // this thread's copies of planes k and k+1 have landed
     __syncthreads();     // ... and everyone's
     const double2 *C = sa + s * kAPlane + me;
@@ -236,10 +247,10 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         u = cadd(u, cmul(d7, azm));
         op = cadd(acc, rmul(vol, u));
       }
-      out[own->w + pn * k] = op;
+      out[az[me] + zp + pn * k] = op;
       e = cmul(phc, op);
       if (hx) {
-        const double c2 = X.e2[i], c3 = X.e3[i], dxi = X.d[i + 1];
+        const double c2 = xe[tx], c3 = xe[kAI + tx], dxi = xe[2 * kAI + tx];
         const double vol = dxi * dyc * z.dc;
         const double2 kx = cur(SK_AX, 0), kp2 = cur(SK_PH, 1), axc = cur(SA_AX, 0);
         const double sum = c2 + c3 + yn4 + yn5 + z.n4 + z.n5;
@@ -253,11 +264,11 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         t = cadd(t, rmul(z.n5, axm));
         const double2 gr = rmul(rdxi, csub(cmul(cur(SA_PH, 1), csub(kp2, kx)), cmul(phc, csub(kpc, kx))));
         const double2 ox = rmul(vol, cadd(t, gr));
-        out[own->x + px * k] = ox;
+        out[axy[me].x + px * k] = ox;
         e = cadd(e, cmul(axc, ox));
       }
       if (hy) {
-        const double c2 = Y.e2[j], c3 = Y.e3[j], dyj = Y.d[j + 1];
+        const double c2 = ye[ty], c3 = ye[kAJ + ty], dyj = ye[2 * kAJ + ty];
         const double vol = dxc * dyj * z.dc;
         const double2 ky = cur(SK_AY, 0), kp2 = cur(SK_PH, kAW), ayc = cur(SA_AY, 0);
         const double sum = c2 + c3 + xn4 + xn5 + z.n4 + z.n5;
@@ -271,7 +282,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         t = cadd(t, rmul(z.n5, aym));
         const double2 gr = rmul(rdyj, csub(cmul(cur(SA_PH, kAW), csub(kp2, ky)), cmul(phc, csub(kpc, ky))));
         const double2 oy = rmul(vol, cadd(t, gr));
-        out[own->y + py * k] = oy;
+        out[axy[me].y + py * k] = oy;
         e = cadd(e, cmul(ayc, oy));
       }
       if (k < nz - 1) {
@@ -289,7 +300,7 @@ static __global__ void __launch_bounds__(kAThreads, 2) k_apply64s(GridDev g, Til
         t = cadd(t, rmul(yn5, cur(SA_AZ, -kAW)));
         const double2 gr = rmul(z.rd, csub(cmul(nxt(SA_PH), csub(kp2, kz)), cmul(phc, csub(kpc, kz))));
         const double2 oz = rmul(vol, cadd(t, gr));
-        out[own->z + pn * k] = oz;
+        out[az[me] + pn * k] = oz;
         e = cadd(e, cmul(azc, oz));
       }
     }
