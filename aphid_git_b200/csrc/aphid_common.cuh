@@ -82,6 +82,9 @@ struct Vals {
   double v[NV];
 };
 
+// The sums over the block, valid in the threads of its first warp (lane c adds
+// the warps' sums of value c: all threads adding all values cost 96 additions and
+// shared-memory reads a thread for the 12 values of a pass).
 template <int NV, int NT>
 __device__ __forceinline__ Vals<NV> block_reduce(Vals<NV> a) {
   __shared__ double sh[NT / 32][NV];
@@ -96,16 +99,18 @@ __device__ __forceinline__ Vals<NV> block_reduce(Vals<NV> a) {
     for (int c = 0; c < NV; c++) sh[w][c] = a.v[c];
   }
   __syncthreads();
-  Vals<NV> r;
-#pragma unroll
-  for (int c = 0; c < NV; c++) {
+  if (threadIdx.x < NV) {
     double s = 0.0;
 #pragma unroll
-    for (int q = 0; q < NT / 32; q++) s += sh[q][c];
-    r.v[c] = s;
+    for (int q = 0; q < NT / 32; q++) s += sh[q][threadIdx.x];
+    sh[0][threadIdx.x] = s;
   }
+  __syncwarp();
+  Vals<NV> r;
+#pragma unroll
+  for (int c = 0; c < NV; c++) r.v[c] = w == 0 ? sh[0][c] : 0.0;
   __syncthreads();
-  return r;  // valid in every thread
+  return r;
 }
 
 // Stores this block's partial, returns true in the last-arriving block of the

@@ -976,7 +976,7 @@ int sweep_alloc(aphid_ctx *ctx, int nsys, bool mixed) {
     CK(cudaMalloc(&ctx->sw_sys, (size_t)nsys * sizeof(SweepSys)));
     CK(cudaMalloc(&ctx->sw_part, (size_t)nsys * ctx->sw_slots * kParts * sizeof(double)));
     // the counters, then the active-system list of the fused passes (k_sw_active)
-    CK(cudaMalloc(&ctx->sw_cnt, ((size_t)CNT_KINDS * nsys + 1 + nsys) * sizeof(unsigned)));
+    CK(cudaMalloc(&ctx->sw_cnt, ((size_t)CNT_KINDS * nsys + 2 + nsys) * sizeof(unsigned)));
     CK(cudaMemsetAsync(ctx->sw_cnt, 0, (size_t)CNT_KINDS * nsys * sizeof(unsigned), ctx->stream));
     if (!ctx->sw_ndone) CK(cudaMalloc(&ctx->sw_ndone, sizeof(int)));
     ctx->sw_nsys = nsys;
@@ -1190,8 +1190,9 @@ void sweep_round_t(aphid_ctx *ctx, const SweepDev &D) {
   const int ring = sizeof(T) == sizeof(double2) ? D.ring64 : D.ring;
   k_sw_dxupd<T, false><<<ps, kStreamThreads, 0, ctx->stream>>>(D);
   k_sw_resid<T><<<st, kOpThreads, 0, ctx->stream>>>(D);
+  // the systems the passes serve; a pass that ends an inner cycle lists them anew
+  k_sw_active<<<1, std::min(1024, (D.nsys + 31) / 32 * 32), 0, ctx->stream>>>(D);
   for (int it = 0; it < ctx->graph_iters; it++) {
-    k_sw_active<<<1, 1024, 0, ctx->stream>>>(D);  // the systems this pass serves
     if (sizeof(T) == sizeof(double2))
       launch_pass64(ctx, D, false);
     else

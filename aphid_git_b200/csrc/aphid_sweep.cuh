@@ -198,7 +198,7 @@ struct SweepDev {
   int timing;                    // fused passes: 1 in timing launches (see k_sw_pass)
   int *work;                     // [2]: next work item, blocks finished (complex64 pass)
   const int *order;              // plane tiles in the order the pass takes them
-  int *active;                   // [1 + nsys]: count, then the systems in their inner cycle (k_sw_active)
+  int *active;                   // [2 + nsys]: count, the systems in their inner cycle, 1 when one has left it since
   // complex128 inner storage (k_sw_pass64): same layouts, double2
   double2 *W64, *P64, *dd64;
   int ring64;
@@ -1250,7 +1250,8 @@ __device__ __noinline__ void pass_scalars(SweepSys *S, const double *T, int ring
 // shared memory; bar, phase: its stage mbarriers and their wait parities.
 template <bool EPS, int CFG, int TS>
 __device__ __forceinline__ void pass_item(const SweepDev &D, const PassMaps &M, int sys, long long tile,
-                                          unsigned char *shm, unsigned long long *bar, unsigned &phase) {
+                                          unsigned char *shm, unsigned long long *bar, unsigned &phase, int *work,
+                                          int &next) {
   using SH = PassShm<EPS, CFG, TS>;
   constexpr int kStages = SH::stages;
   constexpr unsigned kStage = SH::stage, kVecPlane = SH::vec_plane, kSigBytes = SH::sig_bytes;
@@ -1258,7 +1259,10 @@ __device__ __forceinline__ void pass_item(const SweepDev &D, const PassMaps &M, 
                 kKN = PT<TS>::KN;
   float2 *Ub = reinterpret_cast<float2 *>(shm + kStages * kStage);  // [2][4][kPN]
   SweepSys *S = D.sys + sys;
-  if (!D.timing && S->phase != PH_INNER) return;
+  if (!D.timing && S->phase != PH_INNER) {
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(work, 1);
+    return;
+  }
 
   const GridDev &g = D.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -1393,6 +1397,9 @@ __device__ __forceinline__ void pass_item(const SweepDev &D, const PassMaps &M, 
   for (int q = 0; q < kParts; q++) acc[q] = 0.0;
 
   for (int m = k0; m < k1; m++) {
+    // the next item, a plane before it is needed: the counter's round trip runs
+    // under this plane
+    if (m == k1 - 1 && threadIdx.x == 0) next = gridDim.x + atomicAdd(work, 1);
     const int st = (m - k0 + 1) % kStages;
     const float2 *Uc = Ub + ((m - k0) & 1) * 4 * kPN;
     float2 *Un = Ub + ((m - k0 + 1) & 1) * 4 * kPN;
@@ -1524,6 +1531,7 @@ __device__ __forceinline__ void pass_item(const SweepDev &D, const PassMaps &M, 
         S->pslot = (S->pslot + 1) % (D.ring + 1);
       } else {
         pass_scalars(S, tot.v, D.ring);
+        if (D.active && S->phase != PH_INNER) D.active[1 + D.nsys] = 1;
       }
     }
   }
@@ -1533,17 +1541,21 @@ __device__ __forceinline__ void pass_item(const SweepDev &D, const PassMaps &M, 
 // work items from a counter; items of systems that have left their inner
 // cycle cost a counter round trip, two barriers and a phase read each, which
 // on a batch whose last few systems run on alone is a large part of every
-// pass.  So before each pass k_sw_active lists the systems still in their
-// inner cycle, and the pass numbers its items over those only.  Timing
-// launches (and the several-mesh group pass) serve every system.
-static __global__ void __launch_bounds__(1024) k_sw_active(SweepDev D) {
+// pass.  So the systems in their inner cycle are listed, and the pass numbers
+// its items over those only: k_sw_active lists them after a round's outer step,
+// and the last block out of a pass lists them anew when a system's scalar step
+// ended its cycle (a kernel before every pass cost 2 us and a launch gap of a
+// pass of 22 on the smallest meshes).  Timing launches (and the several-mesh
+// group pass) serve every system.  active: [count][systems][stale], see
+// SweepDev.  All threads of a block; phases as L2 has them.
+__device__ __noinline__ void list_active(const SweepSys *sys, int nsys, int *active) {
   __shared__ int s_warp[32], s_base;
   if (threadIdx.x == 0) s_base = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int s0 = 0; s0 < D.nsys; s0 += blockDim.x) {
+  for (int s0 = 0; s0 < nsys; s0 += blockDim.x) {
     const int s = s0 + threadIdx.x;
-    const bool on = s < D.nsys && D.sys[s].phase == PH_INNER;
+    const bool on = s < nsys && *(volatile const int *)&sys[s].phase == PH_INNER;
     const unsigned b = __ballot_sync(0xffffffffu, on);
     if (lane == 0) s_warp[w] = __popc(b);
     __syncthreads();
@@ -1557,11 +1569,15 @@ static __global__ void __launch_bounds__(1024) k_sw_active(SweepDev D) {
       s_base = acc;
     }
     __syncthreads();
-    if (on) D.active[1 + s_warp[w] + __popc(b & ((1u << lane) - 1u))] = s;
+    if (on) active[1 + s_warp[w] + __popc(b & ((1u << lane) - 1u))] = s;
     __syncthreads();
   }
-  if (threadIdx.x == 0) D.active[0] = s_base;
+  if (threadIdx.x == 0) {
+    active[0] = s_base;
+    active[1 + nsys] = 0;
+  }
 }
+static __global__ void __launch_bounds__(1024) k_sw_active(SweepDev D) { list_active(D.sys, D.nsys, D.active); }
 struct ActiveSet {
   const int *list;  // null: every system, in order
   long long n;      // systems served
@@ -1597,16 +1613,25 @@ __device__ __forceinline__ bool pass_block_init(unsigned char *shm, unsigned lon
   }
   return aligned;
 }
-// the last block out of a persistent launch re-arms its work counter
-__device__ __forceinline__ void pass_block_done(int *work) {
+// The last block out of a persistent launch re-arms its work counter and, when
+// a system has left its inner cycle, lists the active ones anew.
+__device__ __forceinline__ void pass_block_done(int *work, const SweepSys *sys, int nsys, int *active) {
+  __shared__ int s_stale;
   if (threadIdx.x == 0) {
+    s_stale = 0;
     __threadfence();
     if (atomicAdd(work + 1, 1) == gridDim.x - 1) {
       work[0] = 0;
       work[1] = 0;
       __threadfence();
+      s_stale = active ? *(volatile const int *)(active + 1 + nsys) : 0;
     }
   }
+  __syncthreads();
+  if (s_stale) list_active(sys, nsys, active);
+}
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *m) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
 
 template <bool EPS, int CFG, int TS>
@@ -1621,20 +1646,24 @@ __global__ void __launch_bounds__(kPThreads, PassShm<EPS, CFG, TS>::blocks) k_sw
   __shared__ int s_sys;
   const bool aligned = pass_block_init<SH::stages>(shm, bar, D.err);
   unsigned phase = 0;  // bit q: parity of the next wait on stage q
+  if (threadIdx.x == 0) prefetch_map(&M.w), prefetch_map(&M.p), prefetch_map(&M.sig);
   const ActiveSet A = active_set(D);
+  // thread 0: the next item; the first ones are the blocks' own, the counter
+  // deals those after them
+  int next = blockIdx.x;
   const long long total = aligned ? D.tp.count() * A.n : 0;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      s_item = atomicAdd(D.work, 1);
-      s_sys = A.sys(s_item, total);
+      s_item = next;
+      s_sys = A.sys(next, total);
     }
     __syncthreads();
     const long long item = s_item;
     if (item >= total) break;
-    pass_item<EPS, CFG, TS>(D, M, s_sys, __ldg(D.order + item / A.n), shm, bar, phase);
+    pass_item<EPS, CFG, TS>(D, M, s_sys, __ldg(D.order + item / A.n), shm, bar, phase, D.work, next);
   }
-  pass_block_done(D.work);
+  pass_block_done(D.work, D.sys, D.nsys, D.timing ? nullptr : D.active);
 }
 
 // Several meshes in one persistent launch (aphid_gpu_sweep_group): the
@@ -1660,9 +1689,10 @@ __global__ void __launch_bounds__(kPThreads, PassShm<EPS, CFG, TS>::blocks) k_sw
   const bool aligned = pass_block_init<SH::stages>(shm, bar, G.D[0].err);  // all meshes in tile shape TS (run_group)
   unsigned phase = 0;
   const long long total = aligned ? G.first[G.n] : 0;
+  int next = blockIdx.x;
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_item = atomicAdd(G.work, 1);
+    if (threadIdx.x == 0) s_item = next;
     __syncthreads();
     const long long item = s_item;
     if (item >= total) break;
@@ -1670,9 +1700,9 @@ __global__ void __launch_bounds__(kPThreads, PassShm<EPS, CFG, TS>::blocks) k_sw
     while (m + 1 < G.n && item >= G.first[m + 1]) m++;
     const long long it = item - G.first[m];
     pass_item<EPS, CFG, TS>(G.D[m], G.M[m], (int)(it % G.D[m].nsys), __ldg(G.D[m].order + it / G.D[m].nsys), shm,
-                            bar, phase);
+                            bar, phase, G.work, next);
   }
-  pass_block_done(G.work);
+  pass_block_done(G.work, nullptr, 0, nullptr);
 }
 
 
@@ -1780,13 +1810,15 @@ __global__ void __launch_bounds__(kPThreads, 1) k_sw_pass64(SweepDev D, const __
   }
   unsigned phase = 0;  // bit q: parity of the next wait on stage q
   __shared__ int s_sys;
+  if (threadIdx.x == 0) prefetch_map(&M.w64);
   const ActiveSet A = active_set(D);
+  int next = blockIdx.x;  // as in k_sw_pass
   const long long total = aligned ? D.tp.count() * A.n : 0;
 
   for (;;) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    s_item = atomicAdd(D.work, 1);
+    s_item = next;
     s_sys = A.sys(s_item, total);
   }
   __syncthreads();
@@ -1795,7 +1827,10 @@ __global__ void __launch_bounds__(kPThreads, 1) k_sw_pass64(SweepDev D, const __
   const int sys = s_sys;
   const long long tile = __ldg(D.order + item / A.n);
   SweepSys *S = D.sys + sys;
-  if (!D.timing && S->phase != PH_INNER) continue;
+  if (!D.timing && S->phase != PH_INNER) {
+    if (threadIdx.x == 0) next = gridDim.x + atomicAdd(D.work, 1);
+    continue;
+  }
 
   const GridDev &g = D.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
@@ -1908,6 +1943,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_sw_pass64(SweepDev D, const __
   for (int q = 0; q < kParts; q++) acc[q] = 0.0;
 
   for (int m = k0; m < k1; m++) {
+    if (m == k1 - 1 && threadIdx.x == 0) next = gridDim.x + atomicAdd(D.work, 1);
     const int st = (m - k0 + 1) % kStages64;
     const double2 *Uc = Ub + ((m - k0) & 1) * 4 * kPN;
     double2 *Un = Ub + ((m - k0 + 1) & 1) * 4 * kPN;
@@ -2038,18 +2074,12 @@ __global__ void __launch_bounds__(kPThreads, 1) k_sw_pass64(SweepDev D, const __
         S->pslot = (S->pslot + 1) % (D.ring64 + 1);
       } else {
         pass_scalars(S, tot.v, D.ring64);
+        if (D.active && S->phase != PH_INNER) D.active[1 + D.nsys] = 1;
       }
     }
   }
   }  // work items
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(D.work + 1, 1) == gridDim.x - 1) {
-      D.work[0] = 0;
-      D.work[1] = 0;
-      __threadfence();
-    }
-  }
+  pass_block_done(D.work, D.sys, D.nsys, D.timing ? nullptr : D.active);
 }
 
 
