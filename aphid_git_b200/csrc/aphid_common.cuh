@@ -122,9 +122,9 @@ __device__ __forceinline__ bool arrive(Vals<NV> blk, double *partials, unsigned 
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int c = 0; c < NV; c++) partials[(size_t)slot * NV + c] = blk.v[c];
-    __threadfence();
-    unsigned t = atomicAdd(counter, 1u);
+      unsigned t = atomicAdd(counter, 1u);
     last = (t == nslots - 1);
+    __threadfence();  // with the barrier: the other blocks' partials, for every thread of the last one
   }
   __syncthreads();
   return last;

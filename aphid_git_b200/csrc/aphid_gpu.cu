@@ -1487,7 +1487,7 @@ int run_batched(aphid_ctx *ctx, const SweepDev &D, bool fused, std::vector<Sweep
   CK(cudaGetLastError());
   nlaunch += 1;
   if ((rc = sweep_graph(ctx, D, fused))) return rc;
-  const long long per_round = 3 + 2LL * ctx->graph_iters + ctx->graph_iters / (fused ? D.ring64 : D.ring);
+  const long long per_round = 4 + (long long)ctx->graph_iters + ctx->graph_iters / (fused ? D.ring64 : D.ring);
   const long long max_rounds = (long long)std::max(1, max_it) / ctx->graph_iters + 2LL * (hs[0].max_outer + 2);
   for (long long round = 0;; round++) {
     CK(cudaMemcpyAsync(ctx->h_ndone, ctx->sw_ndone, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

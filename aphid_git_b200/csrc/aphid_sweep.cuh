@@ -1153,6 +1153,9 @@ __device__ __forceinline__ float2 node_row_c(float2 f, float2 fxp, float2 fxm, f
 // Scalar step at the end of pass n (one thread): epsilon_n, beta_n,
 // rho_{n+1} and delta_{n+1} from the pipelined inner products, then theta,
 // c, eta, kappa, tau and k1 as in src/aphid_qmr.f90:324-372.
+// pull a line towards this SM's L1 ahead of its use (no register, no wait)
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 __device__ __noinline__ void pass_scalars(SweepSys *S, const double *T, int ring) {
   S->cur ^= 1;
   S->pslot = (S->pslot + 1) % (ring + 1);
@@ -1222,6 +1225,133 @@ __device__ __noinline__ void pass_scalars(SweepSys *S, const double *T, int ring
   S->del = del;
   S->k1 = cdiv(rmul(rho, del), e);
   S->vscale = 1.0 / rho;
+}
+
+// The same step by all lanes of one warp, with the sums T in each.  The divisions
+// and square roots (14 and 4, at about 0.2 us each in one thread: 4.3 us of a pass
+// of 22 on the smallest meshes) are done up to four at a time, one per lane: a
+// chain of six divisions and two square roots, 2 us less per pass.  Each is the
+// operation that one thread would do, on the same operands, and which products
+// are fused is written out.  The pass with two blocks per SM keeps the one-thread
+// step: compiled for its 128 registers that one fuses other products, and a
+// solution that starts to round differently moves within the tolerance of its
+// solve; its passes are the long ones (380 us).
+__device__ __forceinline__ double2 cmul_fma(double2 a, double2 b) {
+  return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ double cabs2_fma(double2 a) { return __fma_rn(a.x, a.x, __dmul_rn(a.y, a.y)); }
+struct Smith {  // the ratio and denominator of cdiv(., b)
+  double num, by;  // r = num / by
+  bool wide;       // |b.x| >= |b.y|
+  __device__ __forceinline__ explicit Smith(double2 b) : wide(fabs(b.x) >= fabs(b.y)) {
+    num = wide ? b.y : b.x;
+    by = wide ? b.x : b.y;
+  }
+  __device__ __forceinline__ double den(double2 b, double r) const { return wide ? __fma_rn(b.y, r, b.x) : __fma_rn(b.x, r, b.y); }
+  __device__ __forceinline__ double2 top(double2 a, double r) const {
+    return wide ? make_double2(__fma_rn(a.y, r, a.x), __fma_rn(-a.x, r, a.y))
+                : make_double2(__fma_rn(a.x, r, a.y), __fma_rn(a.y, r, -a.x));
+  }
+};
+__device__ __noinline__ void pass_scalars_warp(SweepSys *S, const double *T, int ring) {
+  const int lane = threadIdx.x & 31;
+  auto pick = [&](double a, double b, double c, double d) { return lane == 0 ? a : lane == 1 ? b : lane == 2 ? c : d; };
+  auto from = [&](double v, int l) { return __shfl_sync(0xffffffffu, v, l); };
+  const double2 e = make_double2(T[0], T[1]);
+  const double A1 = T[2], A3 = T[5];
+  const double2 A2 = make_double2(T[3], T[4]), B1 = make_double2(T[6], T[7]);
+  const double2 B2 = make_double2(T[8], T[9]), B3 = make_double2(T[10], T[11]);
+  const double2 del0 = S->del, eta0 = S->eta;
+  const double c_nm = S->c_nm, rho_n = S->rho_n, theta_nm = S->theta_nm, tau_n = S->tau;
+
+  // beta = e / del; the ratio of the division by e for k1
+  const Smith sd(del0), se(e);
+  double q = pick(sd.num, se.num, 0.0, 0.0) / pick(sd.by, se.by, 1.0, 1.0);
+  const double rd = from(q, 0), re = from(q, 1);
+  const double2 bt = sd.top(e, rd);
+  q = pick(bt.x, bt.y, 0.0, 0.0) / sd.den(del0, rd);
+  const double2 beta = make_double2(from(q, 0), from(q, 1));
+  const double bb = cabs2_fma(beta);
+  double rho2 = __fma_rn(bb, A3, __fma_rn(-2.0, __fma_rn(beta.x, A2.x, __dmul_rn(beta.y, A2.y)), A1));
+  const bool broken = !isfinite(rho2) || !(bb > 0.0);
+  const bool exhausted = !(rho2 > kCancel * A1);  // Krylov space exhausted (or below the expansion's accuracy)
+  if (exhausted) rho2 = 0.0;
+  // rho^2 / c_nm, 1 / rho^2, the ratio of the division for eta
+  const double2 cb = rmul(c_nm, beta);
+  const Smith sb(cb);
+  q = pick(rho2, 1.0, sb.num, 0.0) / pick(c_nm, rho2, sb.by, 1.0);
+  const double t0 = from(q, 0), ir2 = from(q, 1), rb = from(q, 2);
+  const double2 b2 = cmul_fma(beta, B2), b3 = cmul_fma(cmul_fma(beta, beta), B3);
+  const double2 vtv = make_double2(__dadd_rn(__fma_rn(-2.0, b2.x, B1.x), b3.x), __dadd_rn(__fma_rn(-2.0, b2.y, B1.y), b3.y));
+  const double2 del = rmul(ir2, vtv);
+  q = sqrt(pick(rho2, cabs2_fma(csub(B3, del0)), cabs2_fma(del), 1.0));
+  const double rho = from(q, 0), off = from(q, 1), dmag = from(q, 2);
+  // theta, 1 / rho, k1 = rho del / e
+  const double2 kt = se.top(rmul(rho, del), re);
+  const double ke = se.den(e, re);
+  q = pick(t0, 1.0, kt.x, kt.y) / pick(bb, rho, ke, ke);
+  const double theta = from(q, 0), irho = from(q, 1);
+  const double2 k1 = make_double2(from(q, 2), from(q, 3));
+  const double c_n = 1.0 / (1.0 + theta);
+  const double2 et = sb.top(rmul(c_n, rmul(rho_n, cneg(eta0))), rb);
+  q = pick(et.x, et.y, 0.0, 0.0) / sb.den(cb, rb);
+  const double2 eta = make_double2(from(q, 0), from(q, 1));
+  const double kap = theta_nm * c_n, tau = tau_n * sqrt(theta * c_n);
+  __syncwarp();
+  if (lane != 0) return;
+
+  S->cur ^= 1;
+  S->pslot = (S->pslot + 1) % (ring + 1);
+  S->inner_it++;
+  S->total_it++;
+  S->eps = e;
+  if (!finite2(e) || zero2(e) || broken) {  // breakdown: restart from the current x
+    S->phase = PH_OUTER;
+    return;
+  }
+  S->beta = beta;
+  S->rho_np = rho;
+  S->theta_n = theta;
+  S->c_n = c_n;
+  S->eta = eta;
+  S->kap = kap;
+  S->tau = tau;
+  // the solution update of this iteration, d = eta p^_n + kappa d, x += d, for
+  // k_sw_dxupd (the graph flushes the list before it can exceed the ring)
+  const bool update = finite2(eta) && isfinite(kap) && S->npend < kMaxRing;
+  if (update) {
+    S->eta_h[S->npend] = eta;
+    S->kap_h[S->npend] = kap;
+    S->slot_h[S->npend] = S->pslot;
+    S->npend++;
+  }
+  if (exhausted) {
+    S->phase = PH_OUTER;
+    return;
+  }
+  // |v~^T v~ - delta| is measured against ||v~||^2 (about 1), not against
+  // delta, which may be small in complex-symmetric Lanczos without any loss
+  const bool drift = fabs(A3 - 1.0) > kDrift || off > kDrift * A3;
+  if (drift) S->restarts++;
+  bool stall = false;
+  if (S->inner_it - S->win_it >= S->stall_window) {
+    stall = tau > 0.5 * S->tau_win;
+    S->tau_win = tau;
+    S->win_it = S->inner_it;
+  }
+  if (stall) S->restarts++;
+  if (S->escalate && dmag < kDeltaFloor * A3) S->escalated = 1;
+  if (S->escalated || !update || !isfinite(tau) || !finite2(del) || zero2(del) || drift || stall ||
+      tau < S->inner_tol * S->tau0 || S->total_it >= S->max_it) {
+    S->phase = PH_OUTER;
+    return;
+  }
+  S->c_nm = c_n;
+  S->rho_n = rho;
+  S->theta_nm = theta;
+  S->del = del;
+  S->k1 = k1;
+  S->vscale = irho;
 }
 
 // The fused QMR pass (see the file comment).  One persistent block per SM
@@ -1524,15 +1654,17 @@ __device__ __forceinline__ void pass_item(const SweepDev &D, const PassMaps &M, 
   unsigned *cnt = D.cnt + CNT_PASS * D.nsys + sys;
   const unsigned nt = (unsigned)D.tp.count();
   if (arrive<kParts, kPThreads>(blk, part, cnt, (unsigned)tile, nt)) {
+    // the system's scalars on their way to this SM under the last sums
+    if (threadIdx.x * 128 < sizeof(SweepSys)) prefetch_l1(reinterpret_cast<const char *>(S) + threadIdx.x * 128);
     Vals<kParts> tot = final_reduce<kParts, kPThreads>(part, cnt, nt);
-    if (threadIdx.x == 0) {
-      if (D.timing) {
+    if (D.timing) {
+      if (threadIdx.x == 0) {
         S->cur ^= 1;
         S->pslot = (S->pslot + 1) % (D.ring + 1);
-      } else {
-        pass_scalars(S, tot.v, D.ring);
-        if (D.active && S->phase != PH_INNER) D.active[1 + D.nsys] = 1;
       }
+    } else if (threadIdx.x < (SH::blocks == 1 ? 32 : 1)) {
+      SH::blocks == 1 ? pass_scalars_warp(S, tot.v, D.ring) : pass_scalars(S, tot.v, D.ring);
+      if (threadIdx.x == 0 && D.active && S->phase != PH_INNER) D.active[1 + D.nsys] = 1;
     }
   }
 }
@@ -1722,8 +1854,6 @@ struct Pass64Shm {
   static constexpr size_t bytes = kStages64 * (size_t)raw + 2 * (size_t)ubytes + 128;
 };
 
-// pull a line towards this SM's L1 ahead of its use (no register, no wait)
-__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ double2 daxpy(double a, double2 x, double2 y) {
   return make_double2(fma(a, x.x, y.x), fma(a, x.y, y.y));
@@ -2067,15 +2197,17 @@ __global__ void __launch_bounds__(kPThreads, 1) k_sw_pass64(SweepDev D, const __
   unsigned *cnt = D.cnt + CNT_PASS * D.nsys + sys;
   const unsigned nt = (unsigned)D.tp.count();
   if (arrive<kParts, kPThreads>(blk, part, cnt, (unsigned)tile, nt)) {
+    // the system's scalars on their way to this SM under the last sums
+    if (threadIdx.x * 128 < sizeof(SweepSys)) prefetch_l1(reinterpret_cast<const char *>(S) + threadIdx.x * 128);
     Vals<kParts> tot = final_reduce<kParts, kPThreads>(part, cnt, nt);
-    if (threadIdx.x == 0) {
-      if (D.timing) {
+    if (D.timing) {
+      if (threadIdx.x == 0) {
         S->cur ^= 1;
         S->pslot = (S->pslot + 1) % (D.ring64 + 1);
-      } else {
-        pass_scalars(S, tot.v, D.ring64);
-        if (D.active && S->phase != PH_INNER) D.active[1 + D.nsys] = 1;
       }
+    } else if (threadIdx.x < 32) {
+      pass_scalars_warp(S, tot.v, D.ring64);
+      if (threadIdx.x == 0 && D.active && S->phase != PH_INNER) D.active[1 + D.nsys] = 1;
     }
   }
   }  // work items
